@@ -275,6 +275,17 @@ int tt_insert_finalize(const void *accumulator, int32_t complex128, int64_t chan
  * index_put_ accumulates into the output volume directly). */
 int32_t tt_insert_accumulator_layout(const tt_slice_params *p);
 size_t tt_insert_bricked_accumulator_bytes(int64_t d, int64_t h, int64_t w_rfft);
+/* 1 when the float insertion of p's volume (tt_insert_central_slices_rfft_3d)
+ * accumulates into the 2 x 2 x 2-bricked layout. */
+int32_t tt_insert_prefers_bricks(const tt_slice_params *p);
+
+/* Adds channel-interleaved slices (n, channels, h, w/2+1) complex64 to
+ * `channels` bricked float accumulators back to back
+ * (tt_insert_bricked_accumulator_bytes each); every channel gets the weights. */
+int tt_insert_accumulate_bricked(const void *image_rfft, int64_t channels,
+                                 const void *rotation_matrices, void *accumulator,
+                                 const tt_slice_params *p, void *stream);
+
 /* Bricked accumulator -> volume (d, h, w_rfft) complex64 and weights (may be
  * NULL) with the Friedel completion of the x=0 plane, as tt_insert_finalize. */
 int tt_insert_finalize_bricked(const void *accumulator, int64_t d, int64_t h, int64_t w_rfft,
@@ -524,6 +535,57 @@ int tt_backproject_normalize(const void *accumulator, int32_t complex128, int64_
  * grid being that of the (n0, n1, n2) array (backproject.py:80-92). */
 int tt_backproject_finish(const void *volume, int32_t is_f64, int64_t channels, int64_t n0,
                           int64_t n1, int64_t n2, int64_t pad, void *out, void *stream);
+
+/* ---- the real-space wrappers with the transforms included ---------------
+ * float32 maps of box d padded by `pad` on each side to e = d + 2*pad; wr =
+ * e/2 + 1, and L = 2*(wr - 1) the length of the inverse real transform (the
+ * reference's irfftn has no output size).  e and L must be at most 1024 with
+ * prime factors up to 13.  The padding, shifts, sinc^2 weights, scaling and
+ * cropping of project.py:48-92 and backproject.py:48-92 happen in the
+ * transforms' loads and stores; only rows that hold data are read and only
+ * kept samples written. */
+
+/* 1 when the functions below take boxes (d, pad). */
+int32_t tt_transform_supported(int64_t d, int64_t pad);
+
+/* Scratch of one call: `count` volumes (channels) or images. */
+size_t tt_transform_workspace_bytes(int32_t volumes, int64_t count, int64_t d, int64_t pad);
+
+/* Volumes (channels, d, d, d) -> the bricked copies (tt_pack_volume_bricks,
+ * back to back) of the fftshifted rfft of fftshift(pad(volume) * sinc(|f|)^2). */
+int tt_project_volume_bricks(const float *volumes, int64_t channels, int64_t d, int64_t pad,
+                             void *bricks, void *workspace, size_t workspace_bytes, void *stream);
+
+/* Projections (n, channels, d, L - 2*pad) from the bricked copies: central
+ * slices, inverse 2D transforms, crop.  p: n, the padded box as image and
+ * volume shape, the slice options, volume_layout 2. */
+int tt_project_slices(const void *bricks, int64_t channels, const void *rotation_matrices,
+                      int64_t d, int64_t pad, float *images, void *workspace,
+                      size_t workspace_bytes, const tt_slice_params *p, void *stream);
+
+/* Adjoint of the inverse 2D transforms and the crop: gradients of `count`
+ * projections (d, L - 2*pad) -> gradients of their fftshifted slices (e, wr). */
+int tt_project_slices_backward(const float *grad_images, int64_t count, int64_t d, int64_t pad,
+                               void *grad_slices, void *workspace, size_t workspace_bytes,
+                               void *stream);
+
+/* Adjoint of the weighting, padding and 3D transform: gradients of the plain
+ * fftshifted rffts (channels, e, e, wr) -> gradients of the volumes. */
+int tt_project_volume_backward(const void *grad_dft, int64_t channels, int64_t d, int64_t pad,
+                               float *grad_volumes, void *workspace, size_t workspace_bytes,
+                               void *stream);
+
+/* Fftshifted rffts (count, e, wr) of fftshift(pad(images)), images (count, d, d). */
+int tt_backproject_spectra(const float *images, int64_t count, int64_t d, int64_t pad, void *slices,
+                           void *workspace, size_t workspace_bytes, void *stream);
+
+/* Volumes (channels, d, d, L - 2*pad) from the float insertion accumulators
+ * (channels back to back, plain or `bricked`; weights of channel 0): Friedel
+ * completion, division by max(weights, 1), inverse 3D transform, division by
+ * sinc(|f|)^2, crop. */
+int tt_backproject_volume(const void *accumulator, int32_t bricked, int64_t channels, int64_t d,
+                          int64_t pad, float *volumes, void *workspace, size_t workspace_bytes,
+                          void *stream);
 
 #ifdef __cplusplus
 }

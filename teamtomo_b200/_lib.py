@@ -119,6 +119,16 @@ SIGNATURES = {
     "tt_pad_fftshift_2d": ([_vp, _i32, _i64, _i64, _i64, _vp, _vp], _i32),
     "tt_backproject_normalize": ([_vp, _i32, _i64, _i64, _i64, _i64, _vp, _vp], _i32),
     "tt_backproject_finish": ([_vp, _i32, _i64, _i64, _i64, _i64, _i64, _vp, _vp], _i32),
+    "tt_insert_prefers_bricks": ([ctypes.POINTER(SliceParams)], _i32),
+    "tt_insert_accumulate_bricked": ([_vp, _i64, _vp, _vp, ctypes.POINTER(SliceParams), _vp], _i32),
+    "tt_transform_supported": ([_i64, _i64], _i32),
+    "tt_transform_workspace_bytes": ([_i32, _i64, _i64, _i64], _sz),
+    "tt_project_volume_bricks": ([_vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp], _i32),
+    "tt_project_slices": ([_vp, _i64, _vp, _i64, _i64, _vp, _vp, _sz, ctypes.POINTER(SliceParams), _vp], _i32),
+    "tt_project_slices_backward": ([_vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp], _i32),
+    "tt_project_volume_backward": ([_vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp], _i32),
+    "tt_backproject_spectra": ([_vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp], _i32),
+    "tt_backproject_volume": ([_vp, _i32, _i64, _i64, _i64, _vp, _vp, _sz, _vp], _i32),
 }
 
 _lib = None

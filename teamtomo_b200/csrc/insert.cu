@@ -336,6 +336,25 @@ int launch_insert_accumulate(const void* image_rfft, int32_t complex128, const v
     return TT_OK;
 }
 
+// Channel-interleaved images (n, c, h, w/2+1) into c bricked float accumulators
+// back to back, one channel after the other (see launch_insert_accumulate_channels).
+int launch_insert_accumulate_bricked(const float2* img, int64_t channels, const void* rot, float4* acc,
+                                     const tt_slice_params* p, cudaStream_t st) {
+    SliceGeom g = make_geom(*p);
+    g.slice_rows = (int)(channels * g.img_h);
+    const int64_t items = (int64_t)g.n * ((g.img_h + kTileY - 1) / kTileY);
+    if (items > 0x7fffffffLL) return fail(TT_ERR_INVALID, "insert: too many blocks");
+    const size_t bytes = bricked_accumulator_bytes(p);
+    const int nphase = insert_phases(bytes);
+    for (int64_t ch = 0; ch < channels; ch++)
+        for (int ph = 0; ph < nphase; ph++) {
+            insert_accumulate_kernel<float, true><<<(unsigned)items, kTileThreads, 0, st>>>(
+                img + ch * (int64_t)g.img_h * g.wr, rot, acc + ch * (int64_t)(bytes / sizeof(float4)), g, ph, nphase);
+            if (int e = check_launch("insert_accumulate_kernel")) return e;
+        }
+    return TT_OK;
+}
+
 // Channel-interleaved images (n, c, h, w/2+1) into c float accumulators: the
 // single-channel splat once per channel (storage rows per slice: c * h), so
 // each pass reduces into one accumulator with the paired lanes and z-phases
@@ -402,6 +421,24 @@ extern "C" int tt_insert_accumulate(const void* image_rfft, int32_t complex128, 
     return launch_insert_accumulate(image_rfft, complex128, rotation_matrices, accumulator, p, as_stream(stream));
 }
 
+extern "C" int32_t tt_insert_prefers_bricks(const tt_slice_params* p) {
+    return p && !p->deterministic && insert_bricked(p);
+}
+
+extern "C" int tt_insert_accumulate_bricked(const void* image_rfft, int64_t channels, const void* rotation_matrices,
+                                            void* accumulator, const tt_slice_params* p, void* stream) {
+    if (int e = check_insert_params(p)) return e;
+    if (channels < 1 || channels > 4096 || channels * p->img_h > 0x7fffffffLL)
+        return fail(TT_ERR_INVALID, "insert_accumulate_bricked: channels must be in [1, 4096]");
+    if (p->deterministic || p->volume_unshifted)
+        return fail(TT_ERR_INVALID, "insert_accumulate_bricked: a float accumulator of an fftshifted volume");
+    if (p->n == 0) return TT_OK;
+    if (!image_rfft || !rotation_matrices || !accumulator)
+        return fail(TT_ERR_INVALID, "insert_accumulate_bricked: NULL pointer argument");
+    return launch_insert_accumulate_bricked((const float2*)image_rfft, channels, rotation_matrices,
+                                            (float4*)accumulator, p, as_stream(stream));
+}
+
 // The batched insertion's policy: bricked from 64 MB of accumulator while the
 // accumulator fits one z-phase.  Measured on a B200 (batched launch, CTF,
 // best tile shape): 256^3 x 4096 3.77 vs 3.84 ms, 200^3 2.38 vs 2.37 ms (below
@@ -457,17 +494,11 @@ extern "C" int tt_insert_central_slices_rfft_3d(const void* image_rfft, int32_t 
     if (e != cudaSuccess) return fail(TT_ERR_CUDA, "insert: memset: %s", cudaGetErrorString(e));
     if (!complex128 && insert_bricked(p)) {
         // float: the 2 x 2 x 2-bricked accumulator (fewer 128-byte lines per splatted cell)
-        SliceGeom g = make_geom(*p);
-        if (p->n > 0) {
-            const int64_t items = (int64_t)g.n * ((g.img_h + kTileY - 1) / kTileY);
-            if (items > 0x7fffffffLL) return fail(TT_ERR_INVALID, "insert: too many blocks");
-            const int nphase = insert_phases(bricked_accumulator_bytes(p));
-            for (int ph = 0; ph < nphase; ph++) {
-                insert_accumulate_kernel<float, true><<<(unsigned)items, kTileThreads, 0, st>>>(
-                    (const float2*)image_rfft, rotation_matrices, (float4*)workspace, g, ph, nphase);
-                if (int r = check_launch("insert_accumulate_kernel")) return r;
-            }
-        }
+        const SliceGeom g = make_geom(*p);
+        if (p->n > 0)
+            if (int r = launch_insert_accumulate_bricked((const float2*)image_rfft, 1, rotation_matrices,
+                                                         (float4*)workspace, p, st))
+                return r;
         const unsigned rows = (unsigned)(((g.D + 1) / 2) * ((g.H + 1) / 2));
         insert_finalize_bricked_kernel<<<rows, 256, 0, st>>>((const float4*)workspace, (float2*)volume_rfft,
                                                              (float*)weights, g);

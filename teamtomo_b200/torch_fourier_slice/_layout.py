@@ -45,10 +45,19 @@ _MODES = {"plain": PLAIN, "xpairs": XPAIRS, "bricks": BRICKS}
 MIN_PIXELS_PER_VOXEL = 0.5
 
 
+def _mode() -> str:
+    return os.environ.get("TT_VOLUME_LAYOUT", "auto").strip().lower()
+
+
+def automatic() -> bool:
+    """Whether no layout is forced (``TT_VOLUME_LAYOUT``)."""
+    return _mode() == "auto"
+
+
 def choose(n_pixels: int, volume: torch.Tensor) -> int:
     """Layout a call sampling ``n_pixels`` slice pixels from ``volume``
     (complex64, (d, h, w//2+1)) should gather from."""
-    mode = os.environ.get("TT_VOLUME_LAYOUT", "auto").strip().lower()
+    mode = _mode()
     if mode != "auto" and mode not in _MODES:
         raise ValueError(f"TT_VOLUME_LAYOUT must be auto, plain, xpairs or bricks (got {mode!r})")
     if volume.dtype != torch.complex64 or volume.ndim != 3:

@@ -20,7 +20,7 @@ import torch
 
 from .. import _lib
 from . import _wrappers
-from ._params import rotation_arg
+from ._params import rotation_arg, slice_params
 from .slice_insertion import (
     _InsertCentralSlices,
     insert_accumulate,
@@ -31,6 +31,38 @@ from .slice_insertion import (
 
 def _pad_amount(n: int, pad_factor: float) -> int:
     return int((n * (pad_factor - 1.0)) // 2)
+
+
+def _reconstruct(flat, R, c, pad, fftfreq_max, zyx_matrices):
+    """(n * c, d, d) float32 images -> (c, d, d, d') maps with the library's
+    own transforms (csrc/fft.cu) around the insertion."""
+    dev = flat.device
+    d = flat.shape[-1]
+    e = d + 2 * pad
+    wr = e // 2 + 1
+    L = _lib.load()
+    st = _lib.stream_of(dev)
+    params = slice_params(n=R.shape[0], image_shape=(e, e, e), volume=None, rotation=R, fftfreq_max=fftfreq_max,
+                          zyx_matrices=zyx_matrices, vol_dims=(e, e, wr))
+    slices = torch.empty((flat.shape[0], e, wr), dtype=torch.complex64, device=dev)
+    nbytes = max(int(L.tt_transform_workspace_bytes(0, flat.shape[0], d, pad)),
+                 int(L.tt_transform_workspace_bytes(1, c, d, pad)))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    _lib.check(L.tt_backproject_spectra(_lib.ptr(flat), flat.shape[0], d, pad, _lib.ptr(slices), _lib.ptr(ws), nbytes,
+                                        st), "backproject_2d_to_3d")
+    bricked = bool(L.tt_insert_prefers_bricks(params))
+    if bricked:
+        acc = torch.zeros(c * (int(L.tt_insert_bricked_accumulator_bytes(e, e, wr)) // 4), dtype=torch.float32,
+                          device=dev)
+        status = L.tt_insert_accumulate_bricked(_lib.ptr(slices), c, _lib.ptr(R), _lib.ptr(acc), params, st)
+    else:
+        acc = new_accumulator((e, e, e), False, dev, channels=c)
+        status = L.tt_insert_accumulate_multichannel(_lib.ptr(slices), c, _lib.ptr(R), _lib.ptr(acc), params, st)
+    _lib.check(status, "backproject_2d_to_3d")
+    out = torch.empty((c, d, d, 2 * (wr - 1) - 2 * pad), dtype=torch.float32, device=dev)
+    _lib.check(L.tt_backproject_volume(_lib.ptr(acc), int(bricked), c, d, pad, _lib.ptr(out), _lib.ptr(ws), nbytes,
+                                       st), "backproject_2d_to_3d")
+    return out
 
 
 def _backproject(images, rotation_matrices, pad_factor, fftfreq_max, zyx_matrices, channels):
@@ -52,10 +84,15 @@ def _backproject(images, rotation_matrices, pad_factor, fftfreq_max, zyx_matrice
     lead = images.shape[:-3] if channels else images.shape[:-2]
     c = images.shape[-3] if channels else 1
     flat = _lib.dense(images.reshape(-1, d, d))
+    track = torch.is_grad_enabled() and images.requires_grad
+    if (not track and images.dtype == torch.float32 and nrot * c == flat.shape[0] > 0
+            and _lib.load().tt_transform_supported(d, p)):
+        out = _reconstruct(flat, R, c, p, fftfreq_max, zyx_matrices)
+        return out if channels else out[0]
     fft_in = _wrappers.pad_fftshift_2d(flat, p)
     spec = torch.fft.rfftn(fft_in, dim=(-2, -1)).reshape(*lead, c, n, n // 2 + 1)
     spec = spec.reshape(nrot, c, n, n // 2 + 1)
-    if torch.is_grad_enabled() and images.requires_grad:
+    if track:
         vols, weights = _InsertCentralSlices.apply(spec, R, shape, fftfreq_max, zyx_matrices, False, True)
         dft = torch.fft.ifftshift(vols / torch.clamp(weights, min=1.0), dim=(-3, -2))
         real = _wrappers.irfftn_last(dft, 3)

@@ -16,7 +16,8 @@ from collections import OrderedDict
 
 import torch
 
-from . import _wrappers
+from .. import _lib
+from . import _layout, _wrappers
 from ._params import rotation_arg, slice_params
 from .slice_extraction import _ExtractCentralSlices, _ExtractMultichannel
 
@@ -136,15 +137,100 @@ def project_3d_to_2d(
     return _project_eager(volume, rotation_matrices, **kwargs)
 
 
+class _Project(torch.autograd.Function):
+    """(c, d, d, d) float32 maps -> (n, c, d, d') projections with the
+    library's own transforms (csrc/fft.cu): five launches forward.  The
+    backward runs the adjoint passes around the extraction's fused backward;
+    it keeps the bricked copy of the padded rfft when the rotations need a
+    gradient."""
+
+    @staticmethod
+    def forward(ctx, volumes, R, pad, fftfreq_max, zyx_matrices):
+        if not (volumes.is_contiguous() and R.is_contiguous()):
+            raise ValueError("projection needs C-contiguous volumes and rotations")
+        dev = volumes.device
+        c, d, n = volumes.shape[0], volumes.shape[-1], R.shape[0]
+        e = d + 2 * pad
+        wr = e // 2 + 1
+        params = slice_params(n=n, image_shape=(e, e, e), volume=None, rotation=R, fftfreq_max=fftfreq_max,
+                              zyx_matrices=zyx_matrices, rot_tolerance=1e-8, vol_dims=(e, e, wr))
+        params.volume_layout = _layout.BRICKS
+        L = _lib.load()
+        st = _lib.stream_of(dev)
+        bricks = torch.empty(c * (int(L.tt_volume_bricks_bytes(params)) // 8), dtype=torch.complex64, device=dev)
+        nbytes = max(int(L.tt_transform_workspace_bytes(1, c, d, pad)),
+                     int(L.tt_transform_workspace_bytes(0, n * c, d, pad)))
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        out = torch.empty((n, c, d, 2 * (wr - 1) - 2 * pad), dtype=torch.float32, device=dev)
+        _lib.check(L.tt_project_volume_bricks(_lib.ptr(volumes), c, d, pad, _lib.ptr(bricks), _lib.ptr(ws), nbytes,
+                                              st), "project_3d_to_2d")
+        _lib.check(L.tt_project_slices(_lib.ptr(bricks), c, _lib.ptr(R), d, pad, _lib.ptr(out), _lib.ptr(ws), nbytes,
+                                       params, st), "project_3d_to_2d")
+        ctx.meta = (params, c, d, pad)
+        ctx.save_for_backward(R, bricks if ctx.needs_input_grad[1] else None)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad):
+        R, bricks = ctx.saved_tensors
+        params, c, d, pad = ctx.meta
+        want_v, want_r = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+        if not (want_v or want_r):
+            return None, None, None, None, None
+        dev = R.device
+        n, e = R.shape[0], d + 2 * pad
+        wr = e // 2 + 1
+        grad = _lib.dense(grad)
+        L = _lib.load()
+        st = _lib.stream_of(dev)
+        nbytes = max(int(L.tt_transform_workspace_bytes(1, c if want_v else 0, d, pad)),
+                     int(L.tt_transform_workspace_bytes(0, n * c, d, pad)),
+                     int(L.tt_extract_backward_workspace_bytes(params)) if want_r else 0)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        gs = torch.empty((n, c, e, wr), dtype=torch.complex64, device=dev)
+        gdft = torch.zeros((c, e, e, wr), dtype=torch.complex64, device=dev) if want_v else None
+        gr = torch.empty_like(R) if want_r else None
+        _lib.check(L.tt_project_slices_backward(_lib.ptr(grad), n * c, d, pad, _lib.ptr(gs), _lib.ptr(ws), nbytes, st),
+                   "project_3d_to_2d backward")
+        # without d/drotation the backward reads no volume, but wants a pointer to one
+        vol = bricks if bricks is not None else gdft
+        if c == 1:
+            status = L.tt_extract_central_slices_rfft_3d_backward(
+                _lib.ptr(vol), _lib.ptr(R), _lib.ptr(gs), _lib.ptr(gdft), _lib.ptr(gr), _lib.ptr(ws), nbytes, params,
+                st)
+        else:
+            status = L.tt_extract_central_slices_rfft_3d_multichannel_backward(
+                _lib.ptr(vol), c, _lib.ptr(R), _lib.ptr(gs), _lib.ptr(gdft), _lib.ptr(gr), _lib.ptr(ws), nbytes,
+                params, st)
+        _lib.check(status, "project_3d_to_2d backward")
+        gv = None
+        if want_v:
+            gv = torch.empty((c, d, d, d), dtype=torch.float32, device=dev)
+            _lib.check(L.tt_project_volume_backward(_lib.ptr(gdft), c, d, pad, _lib.ptr(gv), _lib.ptr(ws), nbytes, st),
+                       "project_3d_to_2d backward")
+        return gv, gr, None, None, None
+
+
+def _own_transforms(volume, rotations: int, d: int, pad: int) -> bool:
+    """Whether a projection runs on the library's own transforms: single
+    precision, a padded box they take, and no volume layout forced on the
+    gathers."""
+    return (volume.dtype != torch.float64 and volume.is_cuda and rotations > 0 and _layout.automatic()
+            and bool(_lib.load().tt_transform_supported(d, pad)))
+
+
 def _project_eager(volume, rotation_matrices, pad_factor, fftfreq_max, zyx_matrices):
     d = volume.shape[-1]
     p = _pad_amount(volume.shape[-1], pad_factor) if pad_factor > 1.0 else 0
+    R, stack = rotation_arg(rotation_matrices, volume.device)
+    if _own_transforms(volume, R.shape[0], d, p):
+        out = _Project.apply(_lib.dense(volume.to(torch.float32))[None], R, p, fftfreq_max, zyx_matrices)
+        return out.reshape(*stack, *out.shape[-2:])
     n_pad = d + 2 * p
     shape = (n_pad, n_pad, n_pad)
     fft_in = _wrappers.project_prepare(volume, p)  # padded * sinc^2, fftshifted
     # unshifted rfft; cuFFT may hand back a non-contiguous layout
     dft = _slice_source(torch.fft.rfftn(fft_in, dim=(-3, -2, -1)))
-    R, stack = rotation_arg(rotation_matrices, volume.device)
     params = slice_params(n=R.shape[0], image_shape=shape, volume=dft, rotation=R,
                           fftfreq_max=fftfreq_max, zyx_matrices=zyx_matrices,
                           rot_tolerance=1e-8, volume_unshifted=True, slices_unshifted=True)
@@ -171,11 +257,14 @@ def project_3d_to_2d_multichannel(
     if pad_factor < 1.0:
         raise ValueError("pad_factor must be >= 1.0")
     p = _pad_amount(d, pad_factor) if pad_factor > 1.0 else 0
+    R, stack = rotation_arg(rotation_matrices, volume.device)
+    if _own_transforms(volume, R.shape[0], d, p):
+        out = _Project.apply(_lib.dense(volume.to(torch.float32)), R, p, fftfreq_max, zyx_matrices)
+        return out.reshape(*stack, *out.shape[-3:])
     n_pad = d + 2 * p
     shape = (n_pad, n_pad, n_pad)
     fft_in = torch.stack([_wrappers.project_prepare(volume[ch], p) for ch in range(c)])
     dft = _slice_source(torch.fft.rfftn(fft_in, dim=(-3, -2, -1)))
-    R, stack = rotation_arg(rotation_matrices, volume.device)
     params = slice_params(n=R.shape[0], image_shape=shape, volume=dft[0], rotation=R,
                           fftfreq_max=fftfreq_max, zyx_matrices=zyx_matrices,
                           rot_tolerance=1e-8, volume_unshifted=True, slices_unshifted=True)
