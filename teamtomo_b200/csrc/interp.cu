@@ -247,7 +247,235 @@ __global__ void insert3d_bwd_kernel(const T* __restrict__ gimg, const float* __r
     }
 }
 
+// Single-precision trilinear kernels.
+//
+// The generic kernels spend their time in scalar float atomics, one per corner
+// and component, that each reach L2 as a request of their own, and in 64-bit
+// index arithmetic per corner.  Here one voxel index and three strides (32-bit
+// where the image allows it: IDX) address a cell, complex values travel as one
+// 8-byte load or reduction, and the lanes 2j and 2j + 1 of a warp reduce the
+// x-low and the x-high voxel of one point in the same instruction: adjacent
+// voxels, so one L2 request serves both (the L2 takes 197 G requests/s whether
+// one or two such lanes share them).
+//
+// Cell of an inside coordinate: low corner, fractions, strides to the high
+// corners.  A high corner past the last index has fraction 0 and stride 0.
+template <typename IDX>
+struct Cell {
+    IDX base, sz, sy, sx;
+    float tz, ty, tx;
+};
+
+template <typename IDX>
+__device__ __forceinline__ Cell<IDX> cell_of(float cz, float cy, float cx, int D, int H, int W) {
+    const float fz = floorf(cz), fy = floorf(cy), fx = floorf(cx);
+    const int z0 = (int)fz, y0 = (int)fy, x0 = (int)fx;
+    Cell<IDX> k;
+    k.base = ((IDX)z0 * H + y0) * W + x0;
+    k.sz = z0 + 1 < D ? (IDX)H * W : 0;
+    k.sy = y0 + 1 < H ? (IDX)W : 0;
+    k.sx = x0 + 1 < W ? 1 : 0;
+    k.tz = cz - fz;
+    k.ty = cy - fy;
+    k.tx = cx - fx;
+    return k;
+}
+
+__device__ __forceinline__ bool inside3(float cz, float cy, float cx, int D, int H, int W) {
+    return cz >= 0.0f && cz <= (float)(D - 1) && cy >= 0.0f && cy <= (float)(H - 1) && cx >= 0.0f &&
+           cx <= (float)(W - 1);
+}
+
+template <int E>
+struct Vec;
+template <>
+struct Vec<1> {
+    using T = float;
+};
+template <>
+struct Vec<2> {
+    using T = float2;
+};
+__device__ __forceinline__ void vec_fma(float& a, float v, float w) { a = fmaf(v, w, a); }
+__device__ __forceinline__ void vec_fma(float2& a, float2 v, float w) {
+    a.x = fmaf(v.x, w, a.x);
+    a.y = fmaf(v.y, w, a.y);
+}
+__device__ __forceinline__ float vec_mul(float v, float w) { return v * w; }
+__device__ __forceinline__ float2 vec_mul(float2 v, float w) { return make_float2(v.x * w, v.y * w); }
+__device__ __forceinline__ float vec_dot(float a, float b) { return a * b; }
+__device__ __forceinline__ float vec_dot(float2 a, float2 b) { return fmaf(a.x, b.x, a.y * b.y); }
+__device__ __forceinline__ float vec_shfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ float2 vec_shfl(float2 v, int src) {
+    return make_float2(vec_shfl(v.x, src), vec_shfl(v.y, src));
+}
+
+// Weights ((fraction or its complement) products) of corner k: bit 2 z, bit 1 y, bit 0 x.
+template <typename IDX>
+__device__ __forceinline__ IDX corner_offset(const Cell<IDX>& c, int k) {
+    return ((k & 4) ? c.sz : 0) + ((k & 2) ? c.sy : 0) + ((k & 1) ? c.sx : 0);
+}
+
+template <int E, typename IDX>
+__global__ void __launch_bounds__(256)
+sample3d_f32_kernel(const typename Vec<E>::T* __restrict__ img, int C, int D, int H, int W,
+                    const float* __restrict__ coords, int64_t n, typename Vec<E>::T* __restrict__ out) {
+    using V = typename Vec<E>::T;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float cz = __ldcs(coords + i * 3), cy = __ldcs(coords + i * 3 + 1), cx = __ldcs(coords + i * 3 + 2);
+    V* o = out + i * C;
+    if (!inside3(cz, cy, cx, D, H, W)) {
+        for (int ch = 0; ch < C; ch++) o[ch] = V{};
+        return;
+    }
+    const Cell<IDX> k = cell_of<IDX>(cz, cy, cx, D, H, W);
+    const float z0 = 1.0f - k.tz, y0 = 1.0f - k.ty, x0 = 1.0f - k.tx;
+    const IDX plane = (IDX)D * H * W;
+    for (int ch = 0; ch < C; ch++) {
+        const V* p = img + ch * plane + k.base;
+        V v[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) v[c] = __ldg(p + corner_offset(k, c));
+        V acc{};
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            // a corner past the end adds nothing, whatever the voxel its zero stride points at holds
+            const bool there = (!(c & 4) || k.sz) && (!(c & 2) || k.sy) && (!(c & 1) || k.sx);
+            const float w = (((c & 1) ? k.tx : x0) * ((c & 2) ? k.ty : y0)) * ((c & 4) ? k.tz : z0);
+            if (there) vec_fma(acc, v[c], w);
+        }
+        o[ch] = acc;
+    }
+}
+
+template <int E, typename IDX>
+__global__ void __launch_bounds__(256)
+sample3d_f32_bwd_kernel(const typename Vec<E>::T* __restrict__ img, int C, int D, int H, int W,
+                        const float* __restrict__ coords, int64_t n, const typename Vec<E>::T* __restrict__ grad,
+                        typename Vec<E>::T* __restrict__ gimg, float* __restrict__ gcoord) {
+    using V = typename Vec<E>::T;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = i < n;
+    float cz = -1.0f, cy = 0.0f, cx = 0.0f;
+    if (live) {
+        cz = __ldcs(coords + i * 3);
+        cy = __ldcs(coords + i * 3 + 1);
+        cx = __ldcs(coords + i * 3 + 2);
+    }
+    const bool in = live && inside3(cz, cy, cx, D, H, W);
+    if (!in) cz = -1.0f;  // no scatter
+    const IDX plane = (IDX)D * H * W;
+    if (gcoord) {
+        float dz = 0.0f, dy = 0.0f, dx = 0.0f;
+        if (in) {
+            const Cell<IDX> k = cell_of<IDX>(cz, cy, cx, D, H, W);
+            const float z0 = 1.0f - k.tz, y0 = 1.0f - k.ty, x0 = 1.0f - k.tx;
+            for (int ch = 0; ch < C; ch++) {
+                const V g = __ldg(grad + i * C + ch);
+                const V* p = img + ch * plane + k.base;
+                V v[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++) v[c] = __ldg(p + corner_offset(k, c));
+                float d[8];  // Re(conj(G) v), zero past the end
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const bool there = (!(c & 4) || k.sz) && (!(c & 2) || k.sy) && (!(c & 1) || k.sx);
+                    d[c] = there ? vec_dot(g, v[c]) : 0.0f;
+                }
+#pragma unroll
+                for (int b = 0; b < 4; b++) {  // the other two axes' corners
+                    const int zy = (b & 2) * 2 + (b & 1) * 2, zx = (b & 2) * 2 + (b & 1), yx = b;
+                    dx = fmaf(((b & 2) ? k.tz : z0) * ((b & 1) ? k.ty : y0), d[zy + 1] - d[zy], dx);
+                    dy = fmaf(((b & 2) ? k.tz : z0) * ((b & 1) ? k.tx : x0), d[zx + 2] - d[zx], dy);
+                    dz = fmaf(((b & 2) ? k.ty : y0) * ((b & 1) ? k.tx : x0), d[yx + 4] - d[yx], dz);
+                }
+            }
+            if (!coord_grad_passes(cz, D)) dz = 0.0f;
+            if (!coord_grad_passes(cy, H)) dy = 0.0f;
+            if (!coord_grad_passes(cx, W)) dx = 0.0f;
+        }
+        if (live) {
+            __stcs(gcoord + i * 3, dz);
+            __stcs(gcoord + i * 3 + 1, dy);
+            __stcs(gcoord + i * 3 + 2, dx);
+        }
+    }
+    if (!gimg) return;  // the same in every lane
+    const int lane = threadIdx.x & 31, bx = lane & 1;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        const int src = (lane >> 1) + 16 * half;
+        const float pz = vec_shfl(cz, src), py = vec_shfl(cy, src), px = vec_shfl(cx, src);
+        const bool on = pz >= 0.0f;
+        const Cell<IDX> k = cell_of<IDX>(pz, py, px, D, H, W);
+        const float wx = bx ? k.tx : 1.0f - k.tx;
+        for (int ch = 0; ch < C; ch++) {
+            const V g0 = in ? __ldg(grad + i * C + ch) : V{};
+            const V g = vec_shfl(g0, src);
+            V* p = gimg + ch * plane + k.base + bx * k.sx;
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float w = (wx * ((r & 1) ? k.ty : 1.0f - k.ty)) * ((r & 2) ? k.tz : 1.0f - k.tz);
+                const bool there = (!(r & 2) || k.sz) && (!(r & 1) || k.sy) && (!bx || k.sx);
+                if (on && there) atomicAdd(p + (((r & 2) ? k.sz : 0) + ((r & 1) ? k.sy : 0)), vec_mul(g, w));
+            }
+        }
+    }
+}
+
+template <int E, typename WT, typename IDX>
+__global__ void __launch_bounds__(256)
+insert3d_f32_kernel(const typename Vec<E>::T* __restrict__ vals, const float* __restrict__ coords, int64_t n,
+                    typename Vec<E>::T* __restrict__ img, int C, int D, int H, int W, WT* __restrict__ wts) {
+    using V = typename Vec<E>::T;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    float cz = -1.0f, cy = 0.0f, cx = 0.0f;
+    if (i < n) {
+        cz = __ldcs(coords + i * 3);
+        cy = __ldcs(coords + i * 3 + 1);
+        cx = __ldcs(coords + i * 3 + 2);
+    }
+    const bool in = i < n && inside3(cz, cy, cx, D, H, W);
+    if (!in) cz = -1.0f;
+    const IDX plane = (IDX)D * H * W;
+    const int lane = threadIdx.x & 31, bx = lane & 1;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        const int src = (lane >> 1) + 16 * half;
+        const float pz = vec_shfl(cz, src), py = vec_shfl(cy, src), px = vec_shfl(cx, src);
+        const bool on = pz >= 0.0f;
+        const Cell<IDX> k = cell_of<IDX>(pz, py, px, D, H, W);
+        const IDX at = k.base + bx * k.sx;
+        const float wx = bx ? k.tx : 1.0f - k.tx;
+        float w[4];
+        IDX o[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            w[r] = (((r & 2) ? k.tz : 1.0f - k.tz) * ((r & 1) ? k.ty : 1.0f - k.ty)) * wx;
+            o[r] = at + (((r & 2) ? k.sz : 0) + ((r & 1) ? k.sy : 0));
+            if (on && w[r] != 0.0f) atomicAdd(wts + o[r], (WT)w[r]);
+        }
+        for (int ch = 0; ch < C; ch++) {
+            const V v0 = in ? __ldg(vals + i * C + ch) : V{};
+            const V v = vec_shfl(v0, src);
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+                if (on && w[r] != 0.0f) atomicAdd(img + ch * plane + o[r], vec_mul(v, (float)(WT)w[r]));
+        }
+    }
+}
+
 inline unsigned nblocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
+
+// The single-precision trilinear kernels take up to 4096 channels; 8-byte
+// aligned complex images, as torch allocates them.
+inline bool f32_path(int32_t dtype, int32_t nearest, int64_t channels, const void* a, const void* b, const void* c) {
+    const uintptr_t mask = dtype == 2 ? 7 : 3;
+    return (dtype == 0 || dtype == 2) && !nearest && channels <= 4096 &&
+           (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & mask) == 0;
+}
+inline bool idx32(int64_t channels, int64_t d, int64_t h, int64_t w) { return channels * d * h * w < (1LL << 31); }
 
 }  // namespace tt
 
@@ -261,6 +489,18 @@ extern "C" int tt_sample_image_3d(const void* image, int32_t dtype, int64_t chan
         return fail(TT_ERR_INVALID, "sample_image_3d: bad arguments");
     cudaStream_t st = as_stream(stream);
     const unsigned b = nblocks(n, 256);
+    if (f32_path(dtype, nearest, channels, image, out, nullptr)) {
+#define TT_SAMPLE(E, V, IDX)                                                                                       \
+    sample3d_f32_kernel<E, IDX><<<b, 256, 0, st>>>((const V*)image, (int)channels, (int)d, (int)h, (int)w,        \
+                                                   (const float*)coordinates, n, (V*)out)
+        const bool small = idx32(channels, d, h, w);
+        if (dtype == 0 && small) TT_SAMPLE(1, float, int32_t);
+        else if (dtype == 0) TT_SAMPLE(1, float, int64_t);
+        else if (small) TT_SAMPLE(2, float2, int32_t);
+        else TT_SAMPLE(2, float2, int64_t);
+#undef TT_SAMPLE
+        return check_launch("sample3d_f32_kernel");
+    }
     switch (dtype) {
         case 0:
             sample3d_kernel<float, 1><<<b, 256, 0, st>>>((const float*)image, channels, (int)d, (int)h, (int)w,
@@ -292,6 +532,28 @@ extern "C" int tt_insert_into_image_3d(const void* values, int32_t dtype, const 
         return fail(TT_ERR_INVALID, "insert_into_image_3d: bad arguments");
     cudaStream_t st = as_stream(stream);
     const unsigned b = nblocks(n, 256);
+    if (f32_path(dtype, nearest, channels, values, image, nullptr)) {
+#define TT_INSERT(E, V, WT, IDX)                                                                                  \
+    insert3d_f32_kernel<E, WT, IDX><<<b, 256, 0, st>>>((const V*)values, coordinates, n, (V*)image, (int)channels, \
+                                                       (int)d, (int)h, (int)w, (WT*)weights)
+#define TT_INSERT_W(E, V)                                       \
+    if (idx32(channels, d, h, w)) {                             \
+        if (weights_f64) TT_INSERT(E, V, double, int32_t);      \
+        else TT_INSERT(E, V, float, int32_t);                   \
+    } else if (weights_f64) {                                   \
+        TT_INSERT(E, V, double, int64_t);                       \
+    } else {                                                    \
+        TT_INSERT(E, V, float, int64_t);                        \
+    }
+        if (dtype == 0) {
+            TT_INSERT_W(1, float)
+        } else {
+            TT_INSERT_W(2, float2)
+        }
+#undef TT_INSERT_W
+#undef TT_INSERT
+        return check_launch("insert3d_f32_kernel");
+    }
 #define TT_INSERT_CASE(T, E)                                                                                  \
     if (weights_f64)                                                                                          \
         insert3d_kernel<T, E, double><<<b, 256, 0, st>>>((const T*)values, coordinates, n, (T*)image, channels, \
@@ -356,6 +618,19 @@ extern "C" int tt_sample_image_3d_backward(const void* image, int32_t dtype, int
     if (!grad_image && !grad_coordinates) return TT_OK;
     const unsigned b = nblocks(n, 256);
     cudaStream_t st = as_stream(stream);
+    if (f32_path(dtype, nearest, channels, image, grad_out, grad_image)) {
+#define TT_SAMPLE_BWD(E, V, IDX)                                                                                    \
+    sample3d_f32_bwd_kernel<E, IDX><<<b, 256, 0, st>>>((const V*)image, (int)channels, (int)d, (int)h, (int)w,     \
+                                                       (const float*)coordinates, n, (const V*)grad_out,           \
+                                                       (V*)grad_image, (float*)grad_coordinates)
+        const bool small = idx32(channels, d, h, w);
+        if (dtype == 0 && small) TT_SAMPLE_BWD(1, float, int32_t);
+        else if (dtype == 0) TT_SAMPLE_BWD(1, float, int64_t);
+        else if (small) TT_SAMPLE_BWD(2, float2, int32_t);
+        else TT_SAMPLE_BWD(2, float2, int64_t);
+#undef TT_SAMPLE_BWD
+        return check_launch("sample3d_f32_bwd_kernel");
+    }
     switch (dtype) {
         case 0:
             sample3d_bwd_kernel<float, 1><<<b, 256, 0, st>>>((const float*)image, channels, (int)d, (int)h, (int)w,
