@@ -80,8 +80,7 @@ def sample_image_3d(
     batch = coords.shape[:-1]
     c = _lib.dense(coords.reshape(-1, 3).to(_REAL[image.dtype]))
     out = _SampleImage3d.apply(img, c, interpolation == "nearest")
-    out = out.reshape(*batch, C)
-    return out if multi else out[..., 0]
+    return out.reshape(*batch, C) if multi else out.reshape(batch)
 
 
 def insert_into_image_3d(
