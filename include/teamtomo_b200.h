@@ -279,12 +279,12 @@ size_t tt_insert_bricked_accumulator_bytes(int64_t d, int64_t h, int64_t w_rfft)
  * accumulates into the 2 x 2 x 2-bricked layout. */
 int32_t tt_insert_prefers_bricks(const tt_slice_params *p);
 
-/* Adds channel-interleaved slices (n, channels, h, w/2+1) complex64 to
- * `channels` bricked float accumulators back to back
- * (tt_insert_bricked_accumulator_bytes each); every channel gets the weights. */
-int tt_insert_accumulate_bricked(const void *image_rfft, int64_t channels,
-                                 const void *rotation_matrices, void *accumulator,
-                                 const tt_slice_params *p, void *stream);
+/* Adds channel-interleaved slices (n, channels, h, pitch) complex64, w/2+1 of
+ * each row's `pitch` elements used, to `channels` float accumulators back to
+ * back, plain or `bricked`; every channel gets the weights. */
+int tt_insert_accumulate_rows(const void *image_rfft, int64_t channels, int64_t pitch,
+                              const void *rotation_matrices, void *accumulator, int32_t bricked,
+                              const tt_slice_params *p, void *stream);
 
 /* Bricked accumulator -> volume (d, h, w_rfft) complex64 and weights (may be
  * NULL) with the Friedel completion of the x=0 plane, as tt_insert_finalize. */
@@ -539,8 +539,8 @@ int tt_backproject_finish(const void *volume, int32_t is_f64, int64_t channels, 
 /* ---- the real-space wrappers with the transforms included ---------------
  * float32 maps of box d padded by `pad` on each side to e = d + 2*pad; wr =
  * e/2 + 1, and L = 2*(wr - 1) the length of the inverse real transform (the
- * reference's irfftn has no output size).  e and L must be at most 1024 with
- * prime factors up to 13.  The padding, shifts, sinc^2 weights, scaling and
+ * reference's irfftn has no output size).  e and L must be at most 1024 and
+ * products of two to four factors from 2 to 16 and 20 (prime factors up to 13).  The padding, shifts, sinc^2 weights, scaling and
  * cropping of project.py:48-92 and backproject.py:48-92 happen in the
  * transforms' loads and stores; only rows that hold data are read and only
  * kept samples written. */
@@ -548,8 +548,13 @@ int tt_backproject_finish(const void *volume, int32_t is_f64, int64_t channels, 
 /* 1 when the functions below take boxes (d, pad). */
 int32_t tt_transform_supported(int64_t d, int64_t pad);
 
-/* Scratch of one call: `count` volumes (channels) or images. */
-size_t tt_transform_workspace_bytes(int32_t volumes, int64_t count, int64_t d, int64_t pad);
+/* Row length (>= wr, a multiple of 8) of padded half spectra. */
+int64_t tt_transform_row(int64_t d, int64_t pad);
+
+/* Scratch of one call: `count` images (kind 0: tt_project_slices_backward,
+ * tt_backproject_spectra), volumes (1: the *_volume* functions) or projections
+ * (2: tt_project_slices, n * channels). */
+size_t tt_transform_workspace_bytes(int32_t kind, int64_t count, int64_t d, int64_t pad);
 
 /* Volumes (channels, d, d, d) -> the bricked copies (tt_pack_volume_bricks,
  * back to back) of the fftshifted rfft of fftshift(pad(volume) * sinc(|f|)^2). */
@@ -575,7 +580,8 @@ int tt_project_volume_backward(const void *grad_dft, int64_t channels, int64_t d
                                float *grad_volumes, void *workspace, size_t workspace_bytes,
                                void *stream);
 
-/* Fftshifted rffts (count, e, wr) of fftshift(pad(images)), images (count, d, d). */
+/* Fftshifted rffts of fftshift(pad(images)), images (count, d, d): (count, e,
+ * tt_transform_row) complex64, wr of each row's elements written. */
 int tt_backproject_spectra(const float *images, int64_t count, int64_t d, int64_t pad, void *slices,
                            void *workspace, size_t workspace_bytes, void *stream);
 

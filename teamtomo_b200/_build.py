@@ -44,7 +44,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         return LIB
     tmp = LIB + ".tmp"
     cmd = [nvcc_path(), *ARCH_FLAGS, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
-           "-shared", "-cudart", "static", "-o", tmp, *sources()]
+           "-shared", "--threads", "0", "-cudart", "static", "-o", tmp, *sources()]
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
         print(" ".join(cmd), file=sys.stderr)

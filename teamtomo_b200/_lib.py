@@ -120,7 +120,8 @@ SIGNATURES = {
     "tt_backproject_normalize": ([_vp, _i32, _i64, _i64, _i64, _i64, _vp, _vp], _i32),
     "tt_backproject_finish": ([_vp, _i32, _i64, _i64, _i64, _i64, _i64, _vp, _vp], _i32),
     "tt_insert_prefers_bricks": ([ctypes.POINTER(SliceParams)], _i32),
-    "tt_insert_accumulate_bricked": ([_vp, _i64, _vp, _vp, ctypes.POINTER(SliceParams), _vp], _i32),
+    "tt_insert_accumulate_rows": ([_vp, _i64, _i64, _vp, _vp, _i32, ctypes.POINTER(SliceParams), _vp], _i32),
+    "tt_transform_row": ([_i64, _i64], _i64),
     "tt_transform_supported": ([_i64, _i64], _i32),
     "tt_transform_workspace_bytes": ([_i32, _i64, _i64, _i64], _sz),
     "tt_project_volume_bricks": ([_vp, _i64, _i64, _i64, _vp, _vp, _sz, _vp], _i32),

@@ -61,7 +61,7 @@ extract_fwd_kernel(const VT* __restrict__ vol, const void* __restrict__ rot,
     const int iy = ty * kTileY + (threadIdx.x >> 5) * 4 + (lane >> 3);
     if (iy >= g.img_h) return;
     const SliceRow row = slice_row_geom(g, m, iy);
-    float2* orow = out + (s * g.img_h + slice_row(g, iy)) * (int64_t)g.wr;
+    float2* orow = out + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.slice_pitch;
 #pragma unroll UNR
     for (int tx = 0; tx < tx_tiles; tx++) {
         const int ix = tx * kTileX + (lane & 7);
@@ -440,6 +440,16 @@ static int launch_backward(const void* v, const void* rot, const float2* gr, flo
         default:
             return launch_backward_t((const float2*)v, rot, gr, dv, grad_rotation, part, g, st, fixed);
     }
+}
+
+// Slices of a bricked copy, g.slice_rows storage rows of g.slice_pitch elements
+// apart (projections: interleaved channels, padded rows).
+int launch_extract_bricks(const void* bricks, const void* rot, float2* out, const SliceGeom& g, cudaStream_t st) {
+    const int tiles = extract_tiles(g);
+    if ((int64_t)g.n * tiles > 0x7fffffffLL) return fail(TT_ERR_INVALID, "extract: too many blocks");
+    const unsigned nb = (unsigned)((int64_t)g.n * tile_rows(g.img_h));
+    extract_fwd_kernel<<<nb, kExtractThreads, 0, st>>>((const VoxBrick2*)bricks, rot, out, g, tiles);
+    return check_launch("extract_fwd_kernel");
 }
 
 // Bricked copy: voxel (z, y, x), in fftshifted (z, y) order whatever the

@@ -1,19 +1,18 @@
-// Batched 1D Fourier transforms in shared memory, eight at a time per block.
+// Batched 1D Fourier transforms, eight per block, for the kernels of fft.cu.
 //
 // The real-space wrappers pad their inputs to about twice the size and crop
 // their outputs, and every pass of a library transform over the padded arrays
 // moves the zeros and the cropped samples through HBM, with separate passes
 // for the padding, the shifts, the scaling and the layout.  The kernels built
-// on this file (fft.cu) read only the rows that hold data, write only the rows
-// that are kept, and apply shifts, weights, the slice sampling and the volume
-// layout in their loads and stores.
+// on this file read only the rows that hold data, write only the rows that are
+// kept, and apply shifts, weights, the slice sampling and the volume layout in
+// their loads and stores.
 //
-// A block holds eight transforms of length n in a [sample][transform] tile
-// (64-byte rows) and its ping-pong copy: Stockham passes, radix 8, 4, 2, then
-// 3, 5, 7, 11, 13, one butterfly of one transform per thread and step.
-// Consecutive threads take the eight transforms of one sample, so the tile's
-// loads are contiguous; the twiddles are a table of the n-th roots of unity
-// computed once per block.
+// A length n is split into two to four factors of at most 20 (256 = 16 x 16,
+// 320 = 16 x 20, 180 = 12 x 15).  A thread transforms one factor's samples in
+// registers (a Stockham pass); the passes exchange samples through shared
+// memory, so a two-factor length crosses it once, and the first pass can load
+// from and the last store to global memory directly (figures in fft.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -21,54 +20,76 @@
 namespace tt {
 
 constexpr int kFftBatch = 8;          // transforms per block
-constexpr int kFftMaxLength = 1024;   // two tiles of 64 KB
-constexpr int kFftMaxPasses = 10;
+constexpr int kFftMaxLength = 1024;
+constexpr int kFftMaxPasses = 4;
+constexpr int kFftMaxThreads = 256;
 
 struct FftPlan {
     int n;
     int passes;
+    int threads;                     // block size: the widest pass's butterflies, in whole warps
     int radix[kFftMaxPasses];
-    int ns[kFftMaxPasses];           // product of the earlier radices
+    int ns[kFftMaxPasses];           // product of the earlier factors
     uint32_t inv_ns[kFftMaxPasses];  // floor(2^20 / ns) + 1: j / ns = j * inv_ns >> 20 for j * ns < 2^20
+    uint32_t inv_nb[kFftMaxPasses];  // the same for n / radix, used for i < 8 n / radix: i * nb < 2^20
     int step[kFftMaxPasses];         // n / (ns * radix): root stride of the pass
+    int pitched;                     // samples of one transform in the pitched order (padding included)
 };
 
-// Plan of length n; false when n has a prime factor above 13 or is out of range.
-inline bool make_fft_plan(int64_t n, FftPlan& p) {
-    if (n < 2 || n > kFftMaxLength) return false;
-    p.n = (int)n;
-    p.passes = 0;
-    int m = (int)n, twos = 0, ns = 1;
-    auto add = [&](int r) {
-        const int i = p.passes++;
-        p.radix[i] = r;
-        p.ns[i] = ns;
-        p.inv_ns[i] = (1u << 20) / (uint32_t)ns + 1;
-        p.step[i] = (int)n / (ns * r);
-        ns *= r;
-    };
-    while (m % 2 == 0) {
-        m /= 2;
-        twos++;
+constexpr int kFftRadices[] = {20, 16, 15, 14, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+
+// Fewest factors first, then the smallest largest factor; at least two.
+inline bool split_length(int n, int passes, int cap, int* out) {
+    if (passes == 0) return n == 1;
+    for (int r : kFftRadices) {
+        if (r > cap || n % r) continue;
+        out[0] = r;
+        if (split_length(n / r, passes - 1, r, out + 1)) return true;
     }
-    int fours = twos % 3 == 0 ? 0 : (twos % 3 == 2 ? 1 : (twos >= 4 ? 2 : 0));
-    for (int k = 0; k < (twos - 2 * fours) / 3; k++) add(8);
-    for (int k = 0; k < fours; k++) add(4);
-    if (twos == 1) add(2);
-    for (int r : {13, 11, 7, 5, 3})
-        while (m % r == 0) {
-            add(r);
-            m /= r;
-        }
-    return m == 1;
+    return false;
 }
 
-inline size_t fft_smem_bytes(int n) { return (size_t)n * (2 * kFftBatch + 1) * sizeof(float2); }
+// Plan of length n; false when n is not a product of two to four factors in
+// range (a prime factor above 13, a prime, n > 1024).
+inline bool make_fft_plan(int64_t n, FftPlan& p) {
+    if (n < 4 || n > kFftMaxLength) return false;
+    p.n = (int)n;
+    p.passes = 0;
+    int f[kFftMaxPasses];
+    for (int k = 2; k <= kFftMaxPasses && !p.passes; k++)
+        for (int cap = 2; cap <= 20; cap++)
+            if (split_length((int)n, k, cap, f)) {
+                p.passes = k;
+                break;
+            }
+    if (!p.passes) return false;
+    int ns = 1, widest = 0;
+    for (int i = 0; i < p.passes; i++) {
+        const int nb = (int)n / f[i];
+        p.radix[i] = f[i];
+        p.ns[i] = ns;
+        p.inv_ns[i] = (1u << 20) / (uint32_t)ns + 1;
+        p.inv_nb[i] = (1u << 20) / (uint32_t)nb + 1;
+        p.step[i] = (int)n / (ns * f[i]);
+        ns *= f[i];
+        widest = nb > widest ? nb : widest;
+    }
+    p.pitched = (int)n / f[0] * (f[0] | 1);
+    const int t = (widest * kFftBatch + 31) / 32 * 32;
+    p.threads = t < 64 ? 64 : (t > kFftMaxThreads ? kFftMaxThreads : t);
+    return true;
+}
 
-// One thread per sample of a transform, in whole warps.
-inline int fft_threads(int n) {
-    const int t = (n + 31) / 32 * 32;
-    return t < 64 ? 64 : (t > 512 ? 512 : t);
+// Tiles hold eight transforms, [sample][transform] (COLUMNS) or
+// [transform][sample].  Staged samples are in natural order; between passes
+// sample i sits at (i / R) * (R | 1) + i % R, R the first factor, so that the
+// first pass's stores, R apart, fall on different banks and every later access
+// of a butterfly is one base and one stride.
+__device__ __forceinline__ int fft_tile_size(const FftPlan& p) { return p.pitched * kFftBatch; }
+
+// Shared memory: `tiles` tiles and the roots of unity.
+inline size_t fft_smem_bytes(const FftPlan& p, int tiles) {
+    return ((size_t)p.pitched * kFftBatch * tiles + p.n) * sizeof(float2);
 }
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
@@ -77,37 +98,24 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
-// exp(-2 pi i t / n), 0 <= t < n: reduced to the first octant in integers, so
-// the angle handed to sincospi is small and accurate.
+// exp(-2 pi i t / n) (+ when INV), 0 <= t < n: reduced to the first octant in
+// integers, so the angle handed to sincospi is small and accurate.
+template <bool INV>
 __device__ __forceinline__ float2 unit_root(int t, int n) {
-    const int q = (4 * t) / n, r = 4 * t - q * n;  // quarter turns and the rest, r / (4 n) of a turn
+    const int q = (4 * t >= n) + (2 * t >= n) + (4 * t >= 3 * n);  // quarter turns
+    const int r = 4 * t - q * n;                                   // and the rest, r / (4 n) of a turn
     const bool far = 2 * r > n;
     float s, c;
     sincospif((float)(far ? n - r : r) / (float)(2 * n), &s, &c);
-    if (far) {
-        const float x = s;
-        s = c;
-        c = x;
-    }
-    // (c, s) at angle q * pi / 2 + the rest, conjugated
-    switch (q) {
-        case 0: return make_float2(c, -s);
-        case 1: return make_float2(-s, -c);
-        case 2: return make_float2(-c, s);
-        default: return make_float2(s, c);
-    }
+    float2 w = far ? make_float2(s, c) : make_float2(c, s);
+    if (q & 1) w = make_float2(-w.y, w.x);
+    if (q & 2) w = make_float2(-w.x, -w.y);
+    return INV ? w : make_float2(w.x, -w.y);
 }
 
+template <bool INV>
 __device__ __forceinline__ void fft_roots(float2* tw, int n) {
-    for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = unit_root(t, n);
-}
-
-// Tile address of sample k of transform c.  SWZ (tiles that are filled or read
-// along k): the transforms of a sample are permuted so that sixteen
-// consecutive samples of one transform lie in different banks.
-template <bool SWZ>
-__device__ __forceinline__ int fft_at(int k, int c) {
-    return k * kFftBatch + (SWZ ? (c ^ ((k >> 1) & 7)) : c);
+    for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = unit_root<INV>(t, n);
 }
 
 // cos and sin of 2 pi k / R, 0 < k <= R / 2 (k folds to a constant in unrolled code).
@@ -160,8 +168,9 @@ __device__ __forceinline__ float2 turn(float2 a) {
     return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
-// In-register transform of R samples, R odd: pairs (m, R - m) by their sums
-// and differences.
+// ---- transforms of R samples in registers
+
+// R an odd prime: pairs (m, R - m) by their sums and differences.
 template <int R, bool INV>
 struct Dft {
     static __device__ __forceinline__ void run(float2 v[R]) {
@@ -214,73 +223,262 @@ struct Dft<4, INV> {
         v[3] = csub(b, d);
     }
 };
+
+// R = A * B: A transforms of B samples (stride A), twiddles W(a * q), B
+// transforms of A samples.  W(k) multiplies by exp(-+2 pi i k / R).
+template <int A, int B, bool INV, class W>
+__device__ __forceinline__ void dft_split(float2 v[A * B], W twiddle) {
+    float2 t[A][B];
+#pragma unroll
+    for (int a = 0; a < A; a++) {
+#pragma unroll
+        for (int b = 0; b < B; b++) t[a][b] = v[a + A * b];
+        Dft<B, INV>::run(t[a]);
+#pragma unroll
+        for (int q = 1; q < B; q++)
+            if (a) t[a][q] = twiddle(t[a][q], a * q);
+    }
+#pragma unroll
+    for (int q = 0; q < B; q++) {
+        float2 u[A];
+#pragma unroll
+        for (int a = 0; a < A; a++) u[a] = t[a][q];
+        Dft<A, INV>::run(u);
+#pragma unroll
+        for (int a = 0; a < A; a++) v[q + B * a] = u[a];
+    }
+}
+template <bool INV>
+__device__ __forceinline__ float2 by_root(float2 x, float c, float s) {  // exp(-+i angle) from its cos and sin
+    return cmul(x, make_float2(c, INV ? s : -s));
+}
 template <bool INV>
 struct Dft<8, INV> {
     static __device__ __forceinline__ void run(float2 v[8]) {
-        float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-        Dft<4, INV>::run(e);
-        Dft<4, INV>::run(o);
         constexpr float h = 0.70710678118654752f;
-        const float2 w1 = make_float2(h, INV ? h : -h), w3 = make_float2(-h, INV ? h : -h);
-        o[1] = cmul(o[1], w1);
-        o[2] = turn<INV>(o[2]);
-        o[3] = cmul(o[3], w3);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            v[k] = cadd(e[k], o[k]);
-            v[k + 4] = csub(e[k], o[k]);
-        }
+        dft_split<2, 4, INV>(v, [](float2 x, int k) {
+            return k == 1 ? by_root<INV>(x, h, h) : (k == 2 ? turn<INV>(x) : by_root<INV>(x, -h, h));
+        });
+    }
+};
+template <bool INV>
+struct Dft<9, INV> {
+    static __device__ __forceinline__ void run(float2 v[9]) {
+        dft_split<3, 3, INV>(v, [](float2 x, int k) {
+            return k == 1   ? by_root<INV>(x, 0.76604444311897804f, 0.64278760968653933f)
+                   : k == 2 ? by_root<INV>(x, 0.17364817766693035f, 0.98480775301220806f)
+                            : by_root<INV>(x, -0.93969262078590838f, 0.34202014332566873f);  // k == 4
+        });
+    }
+};
+template <bool INV>
+struct Dft<16, INV> {
+    static __device__ __forceinline__ void run(float2 v[16]) {
+        constexpr float h = 0.70710678118654752f, c = 0.92387953251128674f, s = 0.38268343236508977f;
+        dft_split<4, 4, INV>(v, [](float2 x, int k) {
+            return k == 1   ? by_root<INV>(x, c, s)
+                   : k == 2 ? by_root<INV>(x, h, h)
+                   : k == 3 ? by_root<INV>(x, s, c)
+                   : k == 4 ? turn<INV>(x)
+                   : k == 6 ? by_root<INV>(x, -h, h)
+                            : by_root<INV>(x, -c, -s);  // k == 9
+        });
     }
 };
 
-// One Stockham pass of radix R from tile a to tile b.
-template <int R, bool INV, bool SWZ>
-__device__ __forceinline__ void fft_pass(const float2* a, float2* b, const float2* tw, int n, int ns, uint32_t inv_ns,
-                                         int step) {
-    const int nb = n / R;
-    for (int i = threadIdx.x; i < nb * kFftBatch; i += blockDim.x) {
-        const int c = i & (kFftBatch - 1), j = i >> 3;
-        const int k = j - (int)(((uint32_t)j * inv_ns) >> 20) * ns;
-        float2 v[R];
+// R = A * B, A and B coprime: sample (B a + A b) mod R, bin k with k = p mod A,
+// k = q mod B; a two-dimensional transform without twiddles.
+template <int A, int B, bool INV>
+struct DftCoprime {
+    static __host__ __device__ constexpr int inverse(int x, int m) {
+        for (int i = 1; i < m; i++)
+            if (x * i % m == 1) return i;
+        return 0;
+    }
+    static __device__ __forceinline__ void run(float2 v[A * B]) {
+        constexpr int R = A * B, PA = B * inverse(B % A, A), PB = A * inverse(A % B, B);
+        float2 t[A][B];
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = a[fft_at<SWZ>(j + r * nb, c)];
-        if (ns > 1) {
+        for (int a = 0; a < A; a++) {
+#pragma unroll
+            for (int b = 0; b < B; b++) t[a][b] = v[(B * a + A * b) % R];
+            Dft<B, INV>::run(t[a]);
+        }
+#pragma unroll
+        for (int q = 0; q < B; q++) {
+            float2 u[A];
+#pragma unroll
+            for (int a = 0; a < A; a++) u[a] = t[a][q];
+            Dft<A, INV>::run(u);
+#pragma unroll
+            for (int p = 0; p < A; p++) v[(PA * p + PB * q) % R] = u[p];
+        }
+    }
+};
+template <bool INV>
+struct Dft<6, INV> : DftCoprime<2, 3, INV> {};
+template <bool INV>
+struct Dft<10, INV> : DftCoprime<2, 5, INV> {};
+template <bool INV>
+struct Dft<12, INV> : DftCoprime<4, 3, INV> {};
+template <bool INV>
+struct Dft<14, INV> : DftCoprime<2, 7, INV> {};
+template <bool INV>
+struct Dft<15, INV> : DftCoprime<3, 5, INV> {};
+template <bool INV>
+struct Dft<20, INV> : DftCoprime<4, 5, INV> {};
+
+// ---- passes
+//
+// A pass reads butterfly j's samples j + r * nb (nb = n / R) from a source and
+// writes results o + r * ns to a destination.  Sources and destinations give a
+// cursor for one butterfly, then take r.
+
+// A tile in natural order.
+template <bool COLUMNS>
+struct PlainTile {
+    float2* t;
+    int n;
+    __device__ __forceinline__ float2& at(int k, int c) const { return t[COLUMNS ? k * kFftBatch + c : c * n + k]; }
+    struct Cursor {
+        float2* t;
+        int step;
+        __device__ __forceinline__ float2 get(int r) const { return t[r * step]; }
+        __device__ __forceinline__ void put(int r, float2 v) const { t[r * step] = v; }
+    };
+    __device__ __forceinline__ Cursor from(int j, int c, int nb, const FftPlan&) const {
+        return Cursor{&at(j, c), COLUMNS ? nb * kFftBatch : nb};
+    }
+    __device__ __forceinline__ Cursor to(int j, int k, int c, int, const FftPlan& p, int s) const {
+        return Cursor{&at((j - k) * p.radix[s] + k, c), COLUMNS ? p.ns[s] * kFftBatch : p.ns[s]};
+    }
+};
+
+// A tile in the pitched order, between passes.
+template <bool COLUMNS>
+struct PitchedTile {
+    float2* t;
+    using Cursor = typename PlainTile<COLUMNS>::Cursor;
+    __device__ __forceinline__ float2* at(int pos, int c, const FftPlan& p) const {
+        return t + (COLUMNS ? pos * kFftBatch + c : c * p.pitched + pos);
+    }
+    // every pass after the first: nb and ns are multiples of the first factor
+    __device__ __forceinline__ Cursor from(int j, int c, int nb, const FftPlan& p) const {
+        const int R = p.radix[0], pitch = R | 1, q = (int)(((uint32_t)j * p.inv_ns[1]) >> 20);
+        const int rows = (int)(((uint32_t)nb * p.inv_ns[1]) >> 20);
+        return Cursor{at(q * pitch + j - q * R, c, p), rows * pitch * (COLUMNS ? kFftBatch : 1)};
+    }
+    __device__ __forceinline__ Cursor to(int j, int k, int c, int R, const FftPlan& p, int s) const {
+        const int pitch = p.radix[0] | 1;
+        if (s == 0) return Cursor{at(j * pitch, c, p), COLUMNS ? kFftBatch : 1};
+        // results (j - k) * R + k + r * ns
+        const int first = (j - k) * R + k, q = (int)(((uint32_t)first * p.inv_ns[1]) >> 20);
+        const int rows = (int)(((uint32_t)p.ns[s] * p.inv_ns[1]) >> 20);
+        return Cursor{at(q * pitch + first - q * p.radix[0], c, p), rows * pitch * (COLUMNS ? kFftBatch : 1)};
+    }
+};
+
+// Global memory: f.get(x, c) / f.put(x, c, v) with x = (sample - off) mod n, the
+// row or column behind a sample.
+template <class F>
+struct Outside {
+    const F& f;
+    int off, n;
+    struct Cursor {
+        const F& f;
+        int x, step, n, c;
+        __device__ __forceinline__ int where(int r) const {
+            const int y = x + r * step;  // in [0, 2 n)
+            return (int)min((unsigned)y, (unsigned)(y - n));
+        }
+        __device__ __forceinline__ float2 get(int r) const { return f.get(where(r), c); }
+        __device__ __forceinline__ void put(int r, float2 v) const { f.put(where(r), c, v); }
+    };
+    __device__ __forceinline__ int back(int k) const {
+        const int x = k - off;
+        return x < 0 ? x + n : x;
+    }
+    __device__ __forceinline__ Cursor from(int j, int c, int nb, const FftPlan&) const {
+        return Cursor{f, back(j), nb, n, c};
+    }
+    __device__ __forceinline__ Cursor to(int j, int k, int c, int R, const FftPlan& p, int s) const {
+        return Cursor{f, back((j - k) * R + k), p.ns[s], n, c};
+    }
+};
+
+// One Stockham pass of radix R.  Consecutive threads take the eight transforms
+// of one butterfly (COLUMNS) or consecutive butterflies of one transform.
+// Twiddles: the roots of powers r = 1, 2, 4, .. are read, the others are
+// products of at most four of them.
+template <int R, bool INV, bool COLUMNS, bool FIRST, class Src, class Dst>
+__device__ __forceinline__ void fft_pass(const Src& src, const Dst& dst, const float2* tw, const FftPlan& p, int s) {
+    const int nb = p.n / R, ns = FIRST ? 1 : p.ns[s];
+    for (int i = threadIdx.x; i < nb * kFftBatch; i += blockDim.x) {
+        const int c = COLUMNS ? i & (kFftBatch - 1) : (int)(((uint32_t)i * p.inv_nb[s]) >> 20);
+        const int j = COLUMNS ? i >> 3 : i - c * nb;
+        const int k = FIRST ? 0 : j - (int)(((uint32_t)j * p.inv_ns[s]) >> 20) * ns;
+        float2 v[R];
+        const auto in = src.from(j, c, nb, p);
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = in.get(r);
+        if constexpr (!FIRST) {
+            float2 w[R];
+            const int at = k * p.step[s];
 #pragma unroll
             for (int r = 1; r < R; r++) {
-                float2 w = tw[r * k * step];
-                if (INV) w.y = -w.y;
-                v[r] = cmul(v[r], w);
+                const int top = r >= 16 ? 16 : (r >= 8 ? 8 : (r >= 4 ? 4 : (r >= 2 ? 2 : 1)));
+                w[r] = r == top ? tw[r * at] : cmul(w[top], w[r - top]);
+                v[r] = cmul(v[r], w[r]);
             }
         }
         Dft<R, INV>::run(v);
-        const int o = (j - k) * R + k;
+        const auto out = dst.to(j, k, c, R, p, FIRST ? 0 : s);
 #pragma unroll
-        for (int r = 0; r < R; r++) b[fft_at<SWZ>(o + r * ns, c)] = v[r];
+        for (int r = 0; r < R; r++) out.put(r, v[r]);
     }
-    __syncthreads();
 }
 
-// Transforms the tile (the block's eight transforms; a barrier precedes the
-// call) with the exponent's sign - (+ when INV), unscaled; returns the tile
-// that holds the result.
-template <bool INV, bool SWZ>
-__device__ __forceinline__ float2* fft_run(float2* a, float2* b, const float2* tw, const FftPlan& p) {
-    for (int s = 0; s < p.passes; s++) {
-        switch (p.radix[s]) {
-            case 8: fft_pass<8, INV, SWZ>(a, b, tw, p.n, p.ns[s], p.inv_ns[s], p.step[s]); break;
-            case 4: fft_pass<4, INV, SWZ>(a, b, tw, p.n, p.ns[s], p.inv_ns[s], p.step[s]); break;
-            case 2: fft_pass<2, INV, SWZ>(a, b, tw, p.n, p.ns[s], p.inv_ns[s], p.step[s]); break;
-            case 3: fft_pass<3, INV, SWZ>(a, b, tw, p.n, p.ns[s], p.inv_ns[s], p.step[s]); break;
-            case 5: fft_pass<5, INV, SWZ>(a, b, tw, p.n, p.ns[s], p.inv_ns[s], p.step[s]); break;
-            case 7: fft_pass<7, INV, SWZ>(a, b, tw, p.n, p.ns[s], p.inv_ns[s], p.step[s]); break;
-            case 11: fft_pass<11, INV, SWZ>(a, b, tw, p.n, p.ns[s], p.inv_ns[s], p.step[s]); break;
-            default: fft_pass<13, INV, SWZ>(a, b, tw, p.n, p.ns[s], p.inv_ns[s], p.step[s]); break;
-        }
-        float2* t = a;
-        a = b;
-        b = t;
+template <bool INV, bool COLUMNS, bool FIRST, class Src, class Dst>
+__device__ __forceinline__ void fft_any_pass(const Src& src, const Dst& dst, const float2* tw, const FftPlan& p,
+                                             int s) {
+    switch (p.radix[s]) {
+        case 20: fft_pass<20, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 16: fft_pass<16, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 15: fft_pass<15, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 14: fft_pass<14, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 13: fft_pass<13, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 12: fft_pass<12, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 11: fft_pass<11, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 10: fft_pass<10, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 9: fft_pass<9, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 8: fft_pass<8, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 7: fft_pass<7, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 6: fft_pass<6, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 5: fft_pass<5, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 4: fft_pass<4, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        case 3: fft_pass<3, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
+        default: fft_pass<2, INV, COLUMNS, FIRST>(src, dst, tw, p, s); break;
     }
-    return a;
+}
+
+// Transforms the block's eight transforms, exponent sign - (+ when INV),
+// unscaled, from src to dst.  a and b are tiles; b is used from three factors
+// up.  The roots are ready once a barrier has passed since fft_roots; the
+// caller puts one between two calls (and between this call and readers of dst).
+template <bool INV, bool COLUMNS, class Src, class Dst>
+__device__ __forceinline__ void fft_run(const Src& src, const Dst& dst, float2* a, float2* b, const float2* tw,
+                                        const FftPlan& p) {
+    PitchedTile<COLUMNS> from{a}, to{b};
+    fft_any_pass<INV, COLUMNS, true>(src, from, tw, p, 0);
+    __syncthreads();
+    for (int s = 1; s < p.passes - 1; s++) {
+        fft_any_pass<INV, COLUMNS, false>(from, to, tw, p, s);
+        __syncthreads();
+        const PitchedTile<COLUMNS> x = from;
+        from = to;
+        to = x;
+    }
+    fft_any_pass<INV, COLUMNS, false>(from, dst, tw, p, p.passes - 1);
 }
 
 }  // namespace tt

@@ -336,12 +336,13 @@ int launch_insert_accumulate(const void* image_rfft, int32_t complex128, const v
     return TT_OK;
 }
 
-// Channel-interleaved images (n, c, h, w/2+1) into c bricked float accumulators
-// back to back, one channel after the other (see launch_insert_accumulate_channels).
-int launch_insert_accumulate_bricked(const float2* img, int64_t channels, const void* rot, float4* acc,
+// Channel-interleaved images (n, c, h, w/2+1; rows `pitch` elements apart) into c
+// bricked float accumulators back to back, one channel after the other (see launch_insert_accumulate_channels).
+int launch_insert_accumulate_bricked(const float2* img, int64_t channels, int64_t pitch, const void* rot, float4* acc,
                                      const tt_slice_params* p, cudaStream_t st) {
     SliceGeom g = make_geom(*p);
     g.slice_rows = (int)(channels * g.img_h);
+    g.slice_pitch = (int)pitch;
     const int64_t items = (int64_t)g.n * ((g.img_h + kTileY - 1) / kTileY);
     if (items > 0x7fffffffLL) return fail(TT_ERR_INVALID, "insert: too many blocks");
     const size_t bytes = bricked_accumulator_bytes(p);
@@ -349,7 +350,7 @@ int launch_insert_accumulate_bricked(const float2* img, int64_t channels, const 
     for (int64_t ch = 0; ch < channels; ch++)
         for (int ph = 0; ph < nphase; ph++) {
             insert_accumulate_kernel<float, true><<<(unsigned)items, kTileThreads, 0, st>>>(
-                img + ch * (int64_t)g.img_h * g.wr, rot, acc + ch * (int64_t)(bytes / sizeof(float4)), g, ph, nphase);
+                img + ch * (int64_t)g.img_h * pitch, rot, acc + ch * (int64_t)(bytes / sizeof(float4)), g, ph, nphase);
             if (int e = check_launch("insert_accumulate_kernel")) return e;
         }
     return TT_OK;
@@ -362,10 +363,11 @@ int launch_insert_accumulate_bricked(const float2* img, int64_t channels, const 
 // reduced into c accumulators at once and was slower: 2.85 vs 1.97 ms for 2
 // channels, 6.52 vs 3.93 ms for 4 (256^3, 1024 slices).  Every channel gets
 // the weights; readers take them from channel 0.
-int launch_insert_accumulate_channels(const float2* img, int64_t channels, const void* rot, float4* acc,
+int launch_insert_accumulate_channels(const float2* img, int64_t channels, int64_t pitch, const void* rot, float4* acc,
                                       const tt_slice_params* p, cudaStream_t st) {
     SliceGeom g = make_geom(*p);
     g.slice_rows = (int)(channels * g.img_h);
+    g.slice_pitch = (int)pitch;
     const int64_t items = (int64_t)g.n * ((g.img_h + kTileY - 1) / kTileY);
     if (items > 0x7fffffffLL) return fail(TT_ERR_INVALID, "insert multichannel: too many blocks");
     const int64_t vox = (int64_t)g.D * g.H * g.W;
@@ -373,7 +375,7 @@ int launch_insert_accumulate_channels(const float2* img, int64_t channels, const
     for (int64_t ch = 0; ch < channels; ch++)
         for (int ph = 0; ph < nphase; ph++) {
             insert_accumulate_kernel<float><<<(unsigned)items, kTileThreads, 0, st>>>(
-                img + ch * (int64_t)g.img_h * g.wr, rot, acc + ch * vox, g, ph, nphase);
+                img + ch * (int64_t)g.img_h * pitch, rot, acc + ch * vox, g, ph, nphase);
             if (int e = check_launch("insert_accumulate_kernel")) return e;
         }
     return TT_OK;
@@ -425,18 +427,24 @@ extern "C" int32_t tt_insert_prefers_bricks(const tt_slice_params* p) {
     return p && !p->deterministic && insert_bricked(p);
 }
 
-extern "C" int tt_insert_accumulate_bricked(const void* image_rfft, int64_t channels, const void* rotation_matrices,
-                                            void* accumulator, const tt_slice_params* p, void* stream) {
+extern "C" int tt_insert_accumulate_rows(const void* image_rfft, int64_t channels, int64_t pitch,
+                                         const void* rotation_matrices, void* accumulator, int32_t bricked,
+                                         const tt_slice_params* p, void* stream) {
     if (int e = check_insert_params(p)) return e;
     if (channels < 1 || channels > 4096 || channels * p->img_h > 0x7fffffffLL)
-        return fail(TT_ERR_INVALID, "insert_accumulate_bricked: channels must be in [1, 4096]");
+        return fail(TT_ERR_INVALID, "insert_accumulate_rows: channels must be in [1, 4096]");
+    if (pitch < p->img_w / 2 + 1 || pitch > 0x7fffffffLL)
+        return fail(TT_ERR_INVALID, "insert_accumulate_rows: a row holds at least w/2 + 1 elements");
     if (p->deterministic || p->volume_unshifted)
-        return fail(TT_ERR_INVALID, "insert_accumulate_bricked: a float accumulator of an fftshifted volume");
+        return fail(TT_ERR_INVALID, "insert_accumulate_rows: a float accumulator of an fftshifted volume");
     if (p->n == 0) return TT_OK;
     if (!image_rfft || !rotation_matrices || !accumulator)
-        return fail(TT_ERR_INVALID, "insert_accumulate_bricked: NULL pointer argument");
-    return launch_insert_accumulate_bricked((const float2*)image_rfft, channels, rotation_matrices,
-                                            (float4*)accumulator, p, as_stream(stream));
+        return fail(TT_ERR_INVALID, "insert_accumulate_rows: NULL pointer argument");
+    const float2* img = (const float2*)image_rfft;
+    float4* acc = (float4*)accumulator;
+    return bricked ? launch_insert_accumulate_bricked(img, channels, pitch, rotation_matrices, acc, p, as_stream(stream))
+                   : launch_insert_accumulate_channels(img, channels, pitch, rotation_matrices, acc, p,
+                                                       as_stream(stream));
 }
 
 // The batched insertion's policy: bricked from 64 MB of accumulator while the
@@ -496,7 +504,7 @@ extern "C" int tt_insert_central_slices_rfft_3d(const void* image_rfft, int32_t 
         // float: the 2 x 2 x 2-bricked accumulator (fewer 128-byte lines per splatted cell)
         const SliceGeom g = make_geom(*p);
         if (p->n > 0)
-            if (int r = launch_insert_accumulate_bricked((const float2*)image_rfft, 1, rotation_matrices,
+            if (int r = launch_insert_accumulate_bricked((const float2*)image_rfft, 1, g.wr, rotation_matrices,
                                                          (float4*)workspace, p, st))
                 return r;
         const unsigned rows = (unsigned)(((g.D + 1) / 2) * ((g.H + 1) / 2));

@@ -242,7 +242,7 @@ extern "C" int tt_extract_central_slices_rfft_3d_multichannel_backward(
 }
 
 namespace tt {
-int launch_insert_accumulate_channels(const float2* img, int64_t channels, const void* rot, float4* acc,
+int launch_insert_accumulate_channels(const float2* img, int64_t channels, int64_t pitch, const void* rot, float4* acc,
                                       const tt_slice_params* p, cudaStream_t st);  // insert.cu
 }  // namespace tt
 
@@ -260,8 +260,8 @@ extern "C" int tt_insert_accumulate_multichannel(const void* image_rfft, int64_t
     if (!image_rfft || !rotation_matrices || !accumulator)
         return fail(TT_ERR_INVALID, "insert multichannel: NULL pointer argument");
     if (channels * p->img_h > 0x7fffffffLL) return fail(TT_ERR_INVALID, "insert multichannel: too many rows");
-    return launch_insert_accumulate_channels((const float2*)image_rfft, channels, rotation_matrices,
-                                             (float4*)accumulator, p, as_stream(stream));
+    return launch_insert_accumulate_channels((const float2*)image_rfft, channels, p->img_w / 2 + 1,
+                                             rotation_matrices, (float4*)accumulator, p, as_stream(stream));
 }
 
 extern "C" int tt_insert_central_slices_rfft_3d_multichannel_backward(const void* grad_volume, int64_t channels,

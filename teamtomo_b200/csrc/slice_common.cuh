@@ -35,8 +35,10 @@ struct SliceGeom {
     int vol_unshifted;             // volume is the plain rfftn output (no fftshift of z, y)
     int slice_unshifted;           // slices are stored ifftshifted along rows (irfft-ready)
     int vol_layout;                // TT_VOLUME_PLAIN / _XPAIRS / _BRICKS (tt_slice_params.volume_layout)
-    int slice_rows;                // storage rows per slice of the insertion's images
-                                   // (img_h; channels * img_h for channel-interleaved stacks)
+    int slice_rows;                // storage rows per slice of the insertion's images and the
+                                   // extraction's slices (img_h; channels * img_h for
+                                   // channel-interleaved stacks)
+    int slice_pitch;               // elements per storage row of the same (wr, or padded)
     float dcdp0, dcdp1, dcdp2;     // d(array coord)/d(frequency) per axis
 };
 
@@ -73,6 +75,7 @@ __host__ inline SliceGeom make_geom(const tt_slice_params& p) {
     g.slice_unshifted = p.slices_unshifted;
     g.vol_layout = p.volume_layout;
     g.slice_rows = (int)p.img_h;
+    g.slice_pitch = g.wr;
     g.dcdp0 = g.s0 / g.iw0;
     g.dcdp1 = g.s1 / g.iw1;
     g.dcdp2 = 2.0f * g.sx;

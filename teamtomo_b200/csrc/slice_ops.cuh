@@ -432,7 +432,7 @@ __device__ __forceinline__ void insert_point_to(const typename Acc<R>::C* __rest
     const float qx = __fmul_rn((float)ix, g.inv_w);
     if (!insert_pixel_kept(g, qy, qx)) return;
     // issued before the geometry so the load overlaps it
-    const typename Acc<R>::C d = load_slice(img + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.wr + ix);
+    const typename Acc<R>::C d = load_slice(img + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.slice_pitch + ix);
     bool cj;
     InsertCell k;
     if (!insert_cell(g, m, qy, qx, cj, k)) return;
@@ -481,7 +481,7 @@ __device__ __forceinline__ void splat_source(const float2* __restrict__ img, con
     const float qy = shifted_freq(iy, g.img_h, g.inv_h);
     const float qx = __fmul_rn((float)ix, g.inv_w);
     if (!insert_pixel_kept(g, qy, qx)) return;
-    const float2 d = load_slice(img + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.wr + ix);
+    const float2 d = load_slice(img + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.slice_pitch + ix);
     bool cj;
     float ci[3];
     if (!insert_coords(g, m, qy, qx, cj, ci)) return;

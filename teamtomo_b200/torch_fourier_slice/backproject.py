@@ -44,7 +44,8 @@ def _reconstruct(flat, R, c, pad, fftfreq_max, zyx_matrices):
     st = _lib.stream_of(dev)
     params = slice_params(n=R.shape[0], image_shape=(e, e, e), volume=None, rotation=R, fftfreq_max=fftfreq_max,
                           zyx_matrices=zyx_matrices, vol_dims=(e, e, wr))
-    slices = torch.empty((flat.shape[0], e, wr), dtype=torch.complex64, device=dev)
+    row = int(L.tt_transform_row(d, pad))
+    slices = torch.empty((flat.shape[0], e, row), dtype=torch.complex64, device=dev)
     nbytes = max(int(L.tt_transform_workspace_bytes(0, flat.shape[0], d, pad)),
                  int(L.tt_transform_workspace_bytes(1, c, d, pad)))
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
@@ -54,11 +55,10 @@ def _reconstruct(flat, R, c, pad, fftfreq_max, zyx_matrices):
     if bricked:
         acc = torch.zeros(c * (int(L.tt_insert_bricked_accumulator_bytes(e, e, wr)) // 4), dtype=torch.float32,
                           device=dev)
-        status = L.tt_insert_accumulate_bricked(_lib.ptr(slices), c, _lib.ptr(R), _lib.ptr(acc), params, st)
     else:
         acc = new_accumulator((e, e, e), False, dev, channels=c)
-        status = L.tt_insert_accumulate_multichannel(_lib.ptr(slices), c, _lib.ptr(R), _lib.ptr(acc), params, st)
-    _lib.check(status, "backproject_2d_to_3d")
+    _lib.check(L.tt_insert_accumulate_rows(_lib.ptr(slices), c, row, _lib.ptr(R), _lib.ptr(acc), int(bricked), params,
+                                           st), "backproject_2d_to_3d")
     out = torch.empty((c, d, d, 2 * (wr - 1) - 2 * pad), dtype=torch.float32, device=dev)
     _lib.check(L.tt_backproject_volume(_lib.ptr(acc), int(bricked), c, d, pad, _lib.ptr(out), _lib.ptr(ws), nbytes,
                                        st), "backproject_2d_to_3d")

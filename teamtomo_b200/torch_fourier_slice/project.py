@@ -139,7 +139,7 @@ def project_3d_to_2d(
 
 class _Project(torch.autograd.Function):
     """(c, d, d, d) float32 maps -> (n, c, d, d') projections with the
-    library's own transforms (csrc/fft.cu): five launches forward.  The
+    library's own transforms (csrc/fft.cu): seven launches forward.  The
     backward runs the adjoint passes around the extraction's fused backward;
     it keeps the bricked copy of the padded rfft when the rotations need a
     gradient."""
@@ -159,7 +159,7 @@ class _Project(torch.autograd.Function):
         st = _lib.stream_of(dev)
         bricks = torch.empty(c * (int(L.tt_volume_bricks_bytes(params)) // 8), dtype=torch.complex64, device=dev)
         nbytes = max(int(L.tt_transform_workspace_bytes(1, c, d, pad)),
-                     int(L.tt_transform_workspace_bytes(0, n * c, d, pad)))
+                     int(L.tt_transform_workspace_bytes(2, n * c, d, pad)))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
         out = torch.empty((n, c, d, 2 * (wr - 1) - 2 * pad), dtype=torch.float32, device=dev)
         _lib.check(L.tt_project_volume_bricks(_lib.ptr(volumes), c, d, pad, _lib.ptr(bricks), _lib.ptr(ws), nbytes,

@@ -2,7 +2,7 @@
 (csrc/fft.cu) against the same call in float64 torch (projection) and against
 the general path (gradients, reconstruction).
 
-Sizes: every radix (2, 3, 4, 5, 7, 8, 11, 13) alone and mixed, odd padded boxes
+Sizes: factors 2 to 20 in lengths of two and three factors, odd padded boxes
 (whose inverse real transform is one sample shorter), no padding, one and more
 than one block of eight transforms, boxes beyond 48 KB of shared memory, one
 rotation, several channels.
@@ -21,8 +21,8 @@ from helpers import blob_volume, rel_l2, rotations
 
 pytestmark = pytest.mark.gpu
 
-# (d, pad factor): padded 8, 13 -> 12, 26, 22, 27 -> 26, 45 -> 44, 65 -> 64, 98, 104, 128, 180, 256, 320, 49 -> 48
-BOXES = [(4, 2.0), (7, 2.0), (26, 1.0), (22, 1.0), (27, 1.0), (45, 1.0), (33, 2.0), (98, 1.0), (70, 1.5), (64, 2.0),
+# (d, pad factor): padded 8, 25 -> 24, 26, 22, 27 -> 26, 45 -> 44, 65 -> 64, 98, 104, 128, 180, 256, 320, 49 -> 48
+BOXES = [(4, 2.0), (25, 1.0), (26, 1.0), (22, 1.0), (27, 1.0), (45, 1.0), (33, 2.0), (98, 1.0), (70, 1.5), (64, 2.0),
          (90, 2.0), (128, 2.0), (160, 2.0), (33, 1.5)]
 
 
