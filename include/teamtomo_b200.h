@@ -261,11 +261,10 @@ int tt_insert_accumulate(const void *image_rfft, int32_t complex128, const void 
 int tt_insert_finalize(const void *accumulator, int32_t complex128, int64_t channels, int64_t d,
                        int64_t h, int64_t w_rfft, void *volume_rfft, void *weights, void *stream);
 
-/* Accumulator layout for p's volume in the batched float insertion:
- * TT_VOLUME_BRICKS from 64 MB of accumulator up while it fits one z-phase
- * (about 1.1 x the L2; fftshifted volumes), else TT_VOLUME_PLAIN (the
- * one-shot tt_insert_central_slices_rfft_3d bricks every accumulator from
- * 64 MB up, whatever its phases).  A bricked accumulator holds 2 x 2 x 2 voxel bricks of 8
+/* Accumulator layout by the accumulator's size alone (p->n is not used):
+ * TT_VOLUME_BRICKS from 64 MB up while it fits one z-phase (about 1.1 x the
+ * L2; fftshifted float volumes), else TT_VOLUME_PLAIN.  Callers that know
+ * their slices ask tt_insert_prefers_bricks.  A bricked accumulator holds 2 x 2 x 2 voxel bricks of 8
  * (re, im, w, pad) float32 slots (one 128-byte line) in (z, y, x) brick
  * order, x fastest inside a brick, dims rounded up to even
  * (tt_insert_bricked_accumulator_bytes); the splat reduces the eight
@@ -275,8 +274,9 @@ int tt_insert_finalize(const void *accumulator, int32_t complex128, int64_t chan
  * index_put_ accumulates into the output volume directly). */
 int32_t tt_insert_accumulator_layout(const tt_slice_params *p);
 size_t tt_insert_bricked_accumulator_bytes(int64_t d, int64_t h, int64_t w_rfft);
-/* 1 when the float insertion of p's volume (tt_insert_central_slices_rfft_3d)
- * accumulates into the 2 x 2 x 2-bricked layout. */
+/* 1 when the float insertion of p's slices is faster into the bricked layout
+ * (from 200,000 slice pixels and an eighth of a pixel per voxel; the choice of
+ * tt_insert_central_slices_rfft_3d and of the Python batched insertion). */
 int32_t tt_insert_prefers_bricks(const tt_slice_params *p);
 
 /* Adds channel-interleaved slices (n, channels, h, pitch) complex64, w/2+1 of

@@ -204,8 +204,8 @@ def insert_central_slices_rfft_3d_batched(
         cc = _check_ctf(c, n, dev)
         p = slice_params(n=n, image_shape=shape, volume=None, rotation=Rm, fftfreq_max=fftfreq_max,
                          zyx_matrices=zyx_matrices, vol_dims=rfft_shape(shape))
-        # large accumulators are 2 x 2 x 2-bricked (the library's policy, as the one-shot insertion)
-        p.volume_layout = int(L.tt_insert_accumulator_layout(ctypes.byref(p)))
+        # all but small insertions go to 2 x 2 x 2-bricked accumulators (the one-shot insertion's policy)
+        p.volume_layout = _BRICKS if L.tt_insert_prefers_bricks(ctypes.byref(p)) else 0
         if p.volume_layout == _BRICKS:
             d, h, w = rfft_shape(shape)
             acc = torch.zeros(int(L.tt_insert_bricked_accumulator_bytes(d, h, w)) // 4, dtype=torch.float32,

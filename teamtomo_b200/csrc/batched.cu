@@ -64,6 +64,7 @@ batched_slices_kernel(const __grid_constant__ BatchParams bp, unsigned long long
                       int64_t total, int phase, int nphase) {
     constexpr int TY = 256 / TX, RPW = 32 / TX;
     __shared__ float m[9];
+    __shared__ SplatTable tab[INSERT ? 8 : 1];  // one per warp
     __shared__ CtfConst cc;
     __shared__ int64_t cur;
     __shared__ int vsel;
@@ -133,9 +134,11 @@ batched_slices_kernel(const __grid_constant__ BatchParams bp, unsigned long long
                 const int ix = tx * TX + (lane % TX);
                 const bool has_pixel = ix < bv.g.wr && iy < bv.g.img_h;
                 // every lane takes part: lane octets (bricked accumulator) or lane pairs share a pixel
-                if (bv.g.vol_layout == TT_VOLUME_BRICKS)
-                    insert_point_octet(bv.slices, m, bv.acc, bv.g, s, has_pixel, iy, ix, ccp);
-                else
+                if (bv.g.vol_layout == TT_VOLUME_BRICKS) {
+                    float re, im, wscale, c[3];
+                    splat_source(bv.slices, m, bv.g, s, has_pixel, iy, ix, ccp, re, im, wscale, c);
+                    insert_point_octet(bv.acc, bv.g, re, im, wscale, c, tab[threadIdx.x >> 5], true);
+                } else
                     insert_point_paired(bv.slices, m, bv.acc, bv.g, s, has_pixel, iy, ix, ccp);
             }
         }

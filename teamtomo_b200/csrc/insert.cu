@@ -16,12 +16,13 @@
 // same instruction (insert_point_paired): the two voxels usually share an L2
 // sector, so a warp's reductions touch fewer sectors (-15 % time at 256^3).
 //
-// The one-shot entry point (tt_insert_central_slices_rfft_3d) accumulates
-// large float volumes into a 2 x 2 x 2-bricked accumulator instead
+// The one-shot entry point (tt_insert_central_slices_rfft_3d) accumulates all
+// but small calls (insert_bricked) into a 2 x 2 x 2-bricked accumulator instead
 // (accumulator_slot: the eight corners of an even-aligned cell share one
 // 128-byte line; a cell touches 3.4 lines on average instead of 4.5), with
-// the eight corners of a pixel reduced by eight lanes in one instruction
-// (insert_point_octet), split by insert_finalize_bricked_kernel.
+// the eight corners of a pixel reduced by eight lanes in one instruction and
+// shared corners of neighbouring pixels added up before (insert_point_octet),
+// split by insert_finalize_bricked_kernel.
 //
 // Finalize stage: the reference also inserts conj(data)*w at ((d-z)%d, (h-y)%h, 0)
 // for every corner that lands on the x=0 plane except the DC voxel.  Summed
@@ -42,7 +43,7 @@ namespace tt {
 // One block per (slice, row of tiles): the block loads the rotation once and
 // walks the row, skipping the tiles of other z-phases (a few instructions
 // each, so extra phases cost almost nothing).
-template <typename R, bool BRICKED = false>
+template <typename R>
 __global__ void __launch_bounds__(kTileThreads)
 insert_accumulate_kernel(const typename Acc<R>::C* __restrict__ img, const void* __restrict__ rot,
                          typename Acc<R>::T* __restrict__ acc, SliceGeom g, int phase, int nphase) {
@@ -60,12 +61,39 @@ insert_accumulate_kernel(const typename Acc<R>::C* __restrict__ img, const void*
             continue;
         int iy, ix;
         const bool has_pixel = tile_pixel(g, ty * tx_tiles + tx, iy, ix);
-        if constexpr (std::is_same<R, float>::value && BRICKED)
-            insert_point_octet(img, m, acc, g, s, has_pixel, iy, ix);  // every lane takes part
-        else if constexpr (std::is_same<R, float>::value)
+        if constexpr (std::is_same<R, float>::value)
             insert_point_paired(img, m, acc, g, s, has_pixel, iy, ix);  // every lane takes part
         else if (has_pixel)
             insert_point<R>(img, m, acc, g, s, iy, ix);
+    }
+}
+
+// The same into the bricked float accumulator.  Six resident blocks (40
+// registers, no spills): 1.50 against 1.53 ms at five (256^3 x 2048).
+__global__ void __launch_bounds__(kTileThreads, 6)
+insert_bricked_kernel(const float2* __restrict__ img, const void* __restrict__ rot, float4* __restrict__ acc,
+                      SliceGeom g, int phase, int nphase) {
+    __shared__ float m[9];
+    __shared__ SplatTable tab[kTileThreads / 32];
+    const int tx_tiles = tiles_x_of(g.wr);
+    const int rows = (g.img_h + kTileY - 1) / kTileY;
+    const int64_t s = blockIdx.x / rows;
+    const int ty = blockIdx.x - (int)(s * rows);
+    if (threadIdx.x < 9) m[threadIdx.x] = prep_rotation_elem(rot, g.rot_f64, s, threadIdx.x, g, false);
+    __syncthreads();
+    // this thread's pixels share one slice row across the row of tiles
+    const int lane = threadIdx.x & 31;
+    const int iy = ty * kTileY + (threadIdx.x >> 5) * 4 + (lane >> 3);
+    const SliceRow row = slice_row_geom(g, m, iy);
+    const float2* irow = img + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.slice_pitch;
+    for (int tx = 0; tx < tx_tiles; tx++) {
+        if (nphase > 1 && insert_tile_phase(g, m, min(ty * kTileY + kTileY / 2, g.img_h - 1),
+                                            min(tx * kTileX + kTileX / 2, g.wr - 1), nphase) != phase)
+            continue;
+        const int ix = tx * kTileX + (lane & 7);
+        float re, im, wscale, c[3];
+        splat_source_row(irow, m, row, g, iy < g.img_h && ix < g.wr, ix, re, im, wscale, c);
+        insert_point_octet(acc, g, re, im, wscale, c, tab[threadIdx.x >> 5], false);  // every lane takes part
     }
 }
 
@@ -306,15 +334,19 @@ size_t bricked_accumulator_bytes(const tt_slice_params* p) {
     return (size_t)(((p->vol_d + 1) / 2) * ((p->vol_h + 1) / 2) * ((p->vol_w + 1) / 2)) * 8 * sizeof(float4);
 }
 
-// The one-shot float insertion accumulates into the bricked layout from this
-// accumulator size up.  Measured on a B200: 3.86 vs 3.93 ms at 256^3 x 4096
-// slices, 3.21 vs 3.31 ms at 320^3 x 2048, equal at 128^3, and 0.130 vs
-// 0.102 ms at 64^3 x 1000 (where the brick-row finalize's small blocks cost
-// more than the splat saves).
-constexpr size_t kBrickedAccumulatorMinBytes = 64u << 20;
-
+// Whether the float insertion of p's slices accumulates into the bricked
+// layout: from 200,000 slice pixels and an eighth of a pixel per voxel up.
+// Measured on a B200, memset + splat + finalize, plain (x-paired lanes) /
+// bricked (lane octets): 24^3 x 4000 74 / 67 us, 64^3 x 1000 75 / 65, 96^3 x
+// 500 82 / 74, 128^3 x 100 46 / 39, 128^3 x 4096 958 / 781, 200^3 x 2000 1159 /
+// 958, 256^3 x 64 164 / 141, 256^3 x 2048 1964 / 1549, 320^3 x 1024 1732 /
+// 1442; below the line the bricked finalize costs more than the splat saves:
+// 24^3 x 100 7.5 / 9.2, 96^3 x 10 18 / 21, 256^3 x 4 97 / 104, 320^3 x 16 220 /
+// 225.
 bool insert_bricked(const tt_slice_params* p) {
-    return !p->volume_unshifted && bricked_accumulator_bytes(p) >= kBrickedAccumulatorMinBytes;
+    const int64_t pixels = p->n * p->img_h * (p->img_w / 2 + 1);
+    return !p->volume_unshifted && bricks_fit(p) && pixels >= 200000 &&
+           pixels * 8 >= p->vol_d * p->vol_h * p->vol_w;
 }
 
 int launch_insert_accumulate(const void* image_rfft, int32_t complex128, const void* rot, void* acc,
@@ -349,9 +381,9 @@ int launch_insert_accumulate_bricked(const float2* img, int64_t channels, int64_
     const int nphase = insert_phases(bytes);
     for (int64_t ch = 0; ch < channels; ch++)
         for (int ph = 0; ph < nphase; ph++) {
-            insert_accumulate_kernel<float, true><<<(unsigned)items, kTileThreads, 0, st>>>(
+            insert_bricked_kernel<<<(unsigned)items, kTileThreads, 0, st>>>(
                 img + ch * (int64_t)g.img_h * pitch, rot, acc + ch * (int64_t)(bytes / sizeof(float4)), g, ph, nphase);
-            if (int e = check_launch("insert_accumulate_kernel")) return e;
+            if (int e = check_launch("insert_bricked_kernel")) return e;
         }
     return TT_OK;
 }
@@ -447,13 +479,12 @@ extern "C" int tt_insert_accumulate_rows(const void* image_rfft, int64_t channel
                                                        as_stream(stream));
 }
 
-// The batched insertion's policy: bricked from 64 MB of accumulator while the
-// accumulator fits one z-phase.  Measured on a B200 (batched launch, CTF,
-// best tile shape): 256^3 x 4096 3.77 vs 3.84 ms, 200^3 2.38 vs 2.37 ms (below
-// 64 MB), 320^3 x 10000 (two z-phases) 16.1 vs 15.0 ms.
+// By the accumulator's size alone: bricked from 64 MB of accumulator while it
+// fits one z-phase, for callers that do not know their slice counts yet.
 extern "C" int32_t tt_insert_accumulator_layout(const tt_slice_params* p) {
-    if (!p || p->deterministic || !insert_bricked(p)) return TT_VOLUME_PLAIN;
-    return insert_phases(bricked_accumulator_bytes(p)) == 1 ? TT_VOLUME_BRICKS : TT_VOLUME_PLAIN;
+    if (!p || p->deterministic || p->volume_unshifted || !bricks_fit(p)) return TT_VOLUME_PLAIN;
+    const size_t bytes = bricked_accumulator_bytes(p);
+    return bytes >= (64u << 20) && insert_phases(bytes) == 1 ? TT_VOLUME_BRICKS : TT_VOLUME_PLAIN;
 }
 
 extern "C" size_t tt_insert_bricked_accumulator_bytes(int64_t d, int64_t h, int64_t w_rfft) {

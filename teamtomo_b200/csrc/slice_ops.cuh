@@ -270,16 +270,21 @@ __host__ __device__ inline CtfConst make_ctf_const(const tt_ctf_params& p) {
 __device__ __forceinline__ float ctf_value(const CtfConst& k, float qy, float qx) {
     const double y = (double)qy * k.inv_px, x = (double)qx * k.inv_px;
     const double s2 = y * y + x * x;
-    const double inv = 1.0 / sqrt(s2 + 1.1920928955078125e-07);  // torch.finfo(float32).eps
-    const double dot = (y * inv) * k.ay + (x * inv) * k.ax;
-    const double df = (k.defocus - k.astig + 2.0 * dot * dot) * 1e4;  // um -> Angstrom
+    double df = k.defocus * 1e4;  // um -> Angstrom
+    if (k.astig != 0.0) {         // the same for every pixel of an image
+        // (u . a)^2 with u = (y, x) / sqrt(s2 + eps), eps = torch.finfo(float32).eps:
+        // one division instead of a square root and a reciprocal (both in
+        // double: 256^3 x 4096 CTF slices, see batched.cu)
+        const double t = y * k.ay + x * k.ax;
+        df += (2.0 * (t * t) / (s2 + 1.1920928955078125e-07) - k.astig) * 1e4;
+    }
     const double chi = k.k1 * s2 * df + k.k2 * s2 * s2 - k.phase;
-    // the phase is reduced to [-pi, pi] in double (error ~1e-12 at a few
-    // thousand radians); the float sine of the reduced phase is then accurate
-    // to ~1e-7, as the float result, at a fraction of a double sine's cost
-    const double two_pi = 6.283185307179586;
-    const double red = chi - two_pi * rint(chi * (1.0 / two_pi));
-    return -sinf((float)red);
+    // the phase is reduced to half turns in [-1, 1] in double (error ~1e-12 at a
+    // few thousand radians); the float sine of the reduced phase is then
+    // accurate to ~1e-7, as the float result, at a fraction of a double sine's
+    // cost, and sinpi needs no further reduction
+    const double turns = chi * (1.0 / 6.283185307179586);
+    return -sinpif((float)(2.0 * (turns - rint(turns))));
 }
 
 // ---------------------------------------------------------------- insertion
@@ -498,6 +503,35 @@ __device__ __forceinline__ void splat_source(const float2* __restrict__ img, con
     c[2] = ci[2];
 }
 
+// splat_source without a CTF and with the row part of the geometry formed once
+// per thread (slice_row_geom of the thread's slice row): the same operations
+// and roundings.  irow: the storage row's first element.  256^3 x 4096: 2.92
+// against 2.99 ms; the batched kernel, whose registers hold the CTF, loses 3 %
+// with it.
+__device__ __forceinline__ void splat_source_row(const float2* __restrict__ irow, const float* m, const SliceRow& row,
+                                                 const SliceGeom& g, bool has_pixel, int ix, float& dre, float& dim,
+                                                 float& wscale, float c[3]) {
+    dre = 0.f;
+    dim = 0.f;
+    wscale = 1.f;
+    c[0] = -1.f;
+    c[1] = 0.f;
+    c[2] = 0.f;
+    const float qx = __fmul_rn((float)ix, g.inv_w);
+    const bool kept = has_pixel && (!g.has_fmax || __fsqrt_rn(__fadd_rn(row.qy2, __fmul_rn(qx, qx))) <= g.fmax) &&
+                      !(qx == 0.0f && row.qy < 0.0f);
+    if (!kept) return;
+    const float2 d = load_slice(irow + ix);
+    bool cj;
+    float ci[3];
+    if (!insert_coords_row(g, m, row, qx, cj, ci)) return;
+    dre = d.x;
+    dim = cj ? -d.y : d.y;
+    c[0] = ci[0];
+    c[1] = ci[1];
+    c[2] = ci[2];
+}
+
 // Float splat of one source pixel with x-paired lanes into the plain
 // accumulator: lanes 2j and 2j+1 reduce the x-low and the x-high corner of
 // the same pixel in the same instruction (adjacent voxels, usually one
@@ -540,39 +574,94 @@ __device__ __forceinline__ void insert_point_paired(const float2* __restrict__ i
     }
 }
 
+// One warp's pixels on their way from the lane that formed them to the lanes
+// that reduce their corners (insert_point_octet).
+struct SplatTable {
+    float4 data[32];  // re, im, bits of the low corner's slot, bits of the neighbour code
+    float4 cell[32];  // fractions tz, ty, tx, weight scale (0: no pixel)
+};
+
 // Float splat of one source pixel into the 2 x 2 x 2-bricked accumulator
-// (accumulator_slot) with lane octets: lanes 8j..8j+7 reduce the eight
-// corners of one pixel in the same instruction (corner = lane & 7: bit 2 z,
-// bit 1 y, bit 0 x high), four neighbouring pixels of the warp per
-// instruction in eight rounds.  A cell's corners fall on (1.5)^3 128-byte
-// lines on average, which the L2 takes as one request each, against 1.5 lines
-// for each of the four x-paired rows (256^3 x 4096: 3.65 vs 3.82 ms).  Same
-// pixels, corners, weights and values as insert_point_paired; all 32 lanes
-// call it.
-__device__ __forceinline__ void insert_point_octet(const float2* __restrict__ img, const float* m,
-                                                   float4* __restrict__ acc, const SliceGeom& g, int64_t s,
-                                                   bool has_pixel, int iy, int ix, const CtfConst* ctf = nullptr) {
+// (accumulator_slot, fewer than 2^32 slots) with lane octets: lanes 8j..8j+7
+// reduce the eight corners of one pixel in the same instruction (corner =
+// lane & 7: bit 2 z, bit 1 y, bit 0 x high), four neighbouring pixels of a
+// slice row per instruction in eight rounds.  A cell's corners fall on (1.5)^3
+// 128-byte lines on average, which leave the SM as one request each.
+//
+// The reductions are bound by the SM's request port to the L2 (82 % busy with
+// one reduction per pixel and corner, at 60 % of the issue slots), so corners
+// that two pixels share are added up first: the outer pixels of the four hand
+// the corners that fall on their inner neighbour's cell to it (lanes 0 -> 1
+// and 3 -> 2; the shared voxels follow from the two cells' offset, at most one
+// voxel per axis).  256^3 x 2048 slices: 21 % fewer reduced sectors, 1.50 ms
+// against 1.79; 128^3 x 4096: 0.77 against 0.88; 320^3 x 1024: 1.41 against
+// 1.60.  The pixel records go through shared memory (two 16-byte broadcasts a
+// round instead of seven shuffles).  Handing on from 1 to 2 as well takes
+// another 15 % of the sectors but 22 more instructions a round, and the kernel
+// is then bound by issue: 1.76 ms.
+//
+// dre, dim, wscale and c are the lane's pixel (splat_source; ctf: it may have a CTF);
+// same corners and weights ((fz * fy) * fx) as insert_point.  All 32 lanes of
+// the warp call it, with the warp's own table.
+__device__ __forceinline__ void insert_point_octet(float4* __restrict__ acc, const SliceGeom& g, float dre, float dim,
+                                                   float wscale, const float c[3], SplatTable& tab, bool ctf) {
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, corner = lane & 7;
-    const int bz = corner >> 2, by = (corner >> 1) & 1, bx = corner & 1;
-    float dre, dim, wscale, c[3];
-    splat_source(img, m, g, s, has_pixel, iy, ix, ctf, dre, dim, wscale, c);
+    const int lane = threadIdx.x & 31, corner = lane & 7, p = lane >> 3;
+    const uint32_t bh = (uint32_t)(g.H + 1) >> 1, bw = (uint32_t)(g.W + 1) >> 1;
+    {
+        const bool on = c[0] >= 0.0f;
+        const float fz = floorf(c[0]), fy = floorf(c[1]), fx = floorf(c[2]);
+        // a lane without a pixel: a cell far from every other, all of its corners zero
+        const int z0 = on ? (int)fz : -0x10000, y0 = (int)fy, x0 = (int)fx;
+        const uint32_t slot = (((uint32_t)z0 >> 1) * bh + ((uint32_t)y0 >> 1)) * bw * 8u + ((uint32_t)x0 >> 1) * 8u +
+                              (((uint32_t)z0 & 1u) << 2) + (((uint32_t)y0 & 1u) << 1) + ((uint32_t)x0 & 1u);
+        // neighbour code: corner k of this cell is corner k + D of the neighbour's;
+        // bits 0-7 the corners for which it exists, bits 8-11 D + 8
+        const int dz = z0 - __shfl_xor_sync(full, z0, 1), dy = y0 - __shfl_xor_sync(full, y0, 1),
+                  dx = x0 - __shfl_xor_sync(full, x0, 1);
+        const int pair_on = __shfl_xor_sync(full, (int)on, 1);  // every lane shuffles
+        const bool both = on && pair_on;
+        const int mz = dz == 0 ? 0xff : (dz == 1 ? 0x0f : (dz == -1 ? 0xf0 : 0));
+        const int my = dy == 0 ? 0xff : (dy == 1 ? 0x33 : (dy == -1 ? 0xcc : 0));
+        const int mx = dx == 0 ? 0xff : (dx == 1 ? 0x55 : (dx == -1 ? 0xaa : 0));
+        const int code = (both ? mz & my & mx : 0) | (((dz * 4 + dy * 2 + dx + 8) & 15) << 8);
+        __syncwarp();  // the previous call's reads
+        tab.data[lane] = make_float4(dre, dim, __uint_as_float(on ? slot : 0u), __int_as_float(code));
+        tab.cell[lane] = on ? make_float4(c[0] - fz, c[1] - fy, c[2] - fx, wscale) : make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+    }
+    // per axis: fraction t -> t (high corner) or 1 - t (low), both exact
+    const float az = (corner & 4) ? 1.0f : -1.0f, bz = (corner & 4) ? 0.0f : 1.0f;
+    const float ay = (corner & 2) ? 1.0f : -1.0f, by = (corner & 2) ? 0.0f : 1.0f;
+    const float ax = (corner & 1) ? 1.0f : -1.0f, bx = (corner & 1) ? 0.0f : 1.0f;
+    // slots from the low corner to this lane's, from an even / odd coordinate
+    const uint32_t ez = (corner & 4) ? 4u : 0u, oz = (corner & 4) ? bh * bw * 8u - 4u : 0u;
+    const uint32_t ey = (corner & 2) ? 2u : 0u, oy = (corner & 2) ? bw * 8u - 2u : 0u;
+    const uint32_t ex = (corner & 1) ? 1u : 0u, ox = (corner & 1) ? 7u : 0u;
+    const bool inner = p == 1 || p == 2;
+    const int other = ((p ^ 1) << 3) + corner - 8;
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-        const int src = 4 * r + (lane >> 3);
-        const float sre = __shfl_sync(full, dre, src), sim = __shfl_sync(full, dim, src);
-        const float sws = ctf ? __shfl_sync(full, wscale, src) : 1.0f;
-        float sc[3];
-#pragma unroll
-        for (int a = 0; a < 3; a++) sc[a] = __shfl_sync(full, c[a], src);
-        if (sc[0] < 0.0f) continue;
-        InsertCell k;
-        cell_at(sc, k);
-        const float w = ((bz ? k.tz : 1.0f - k.tz) * (by ? k.ty : 1.0f - k.ty)) * (bx ? k.tx : 1.0f - k.tx);
-        if (w != 0.0f) {
-            const int z = bz ? k.iz1 : k.iz0, y = by ? k.iy1 : k.iy0, x = bx ? k.ix1 : k.ix0;
-            acc_add(acc + accumulator_slot(g, z, y, x), sre * w, sim * w, w * sws);
+        const float4 d = tab.data[4 * r + p], f = tab.cell[4 * r + p];
+        const uint32_t base = __float_as_uint(d.z);
+        const int code = __float_as_int(d.w);
+        const float w = (fmaf(f.x, az, bz) * fmaf(f.y, ay, by)) * fmaf(f.z, ax, bx);
+        const uint32_t slot = base + ((base & 4u) ? oz : ez) + ((base & 2u) ? oy : ey) + ((base & 1u) ? ox : ex);
+        // a corner of zero weight adds nothing, whatever the data
+        float re = w != 0.0f ? d.x * w : 0.0f, im = w != 0.0f ? d.y * w : 0.0f, wt = w * f.w;
+        const bool shared = (code >> corner) & 1;
+        const int from = other + ((code >> 8) & 15);
+        const float ore = __shfl_sync(full, re, from), oim = __shfl_sync(full, im, from),
+                    owt = __shfl_sync(full, wt, from);
+        if (shared && inner) {
+            re += ore;
+            im += oim;
+            wt += owt;
         }
+        // with a CTF the weight can vanish where the data do not
+        const bool any = ctf ? ((__float_as_uint(re) | __float_as_uint(im) | __float_as_uint(wt)) & 0x7fffffffu) != 0
+                             : wt != 0.0f;
+        if (any && (inner || !shared)) acc_add(acc + slot, re, im, wt);
     }
 }
 
