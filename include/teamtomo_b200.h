@@ -484,6 +484,19 @@ int tt_insert_into_image_3d(const void *values, int32_t dtype, const float *coor
                             void *image, int64_t channels, int64_t d, int64_t h, int64_t w,
                             void *weights, int32_t weights_f64, int32_t nearest, void *stream);
 
+/* The same with scratch: from one point per voxel (single channel, single
+ * precision, trilinear, float32 weights) the points go to a bricked
+ * accumulator first, which is then added to image and weights.  The bytes are
+ * 0 where tt_insert_into_image_3d's direct splat is used. */
+size_t tt_insert_into_image_3d_workspace_bytes(int32_t dtype, int64_t n, int64_t channels, int64_t d,
+                                               int64_t h, int64_t w, int32_t weights_f64,
+                                               int32_t nearest);
+int tt_insert_into_image_3d_workspace(const void *values, int32_t dtype, const float *coordinates,
+                                      int64_t n, void *image, int64_t channels, int64_t d,
+                                      int64_t h, int64_t w, void *weights, int32_t weights_f64,
+                                      int32_t nearest, void *workspace, size_t workspace_bytes,
+                                      void *stream);
+
 /* Affine resampling: out (n_matrices, od, oh, ow, channels) of the image's
  * dtype = image sampled at M (z, y, x, 1) for every output voxel (z, y, x),
  * matrices_zyx (n_matrices, 4, 4) float32 already in zyx order; coordinates in

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "capi_util.cuh"
+#include "slice_ops.cuh"
 
 namespace tt {
 
@@ -466,6 +467,63 @@ insert3d_f32_kernel(const typename Vec<E>::T* __restrict__ vals, const float* __
     }
 }
 
+// The splat of many points through a bricked accumulator: one (re, im, weight,
+// 0) float4 per corner by the slice insertion's lane octets
+// (insert_point_octet: corners that neighbouring points share are added up
+// before the reduction) instead of two reductions per corner into image and
+// weights, then one pass that adds the accumulator to both.
+template <int E>
+__global__ void __launch_bounds__(256, 6)
+splat_bricked_kernel(const typename Vec<E>::T* __restrict__ vals, const float* __restrict__ coords, int64_t n,
+                     float4* __restrict__ acc, SliceGeom g) {
+    __shared__ SplatTable tab[8];
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    float c[3] = {-1.0f, 0.0f, 0.0f}, re = 0.0f, im = 0.0f;
+    if (i < n) {
+        const float cz = __ldcs(coords + i * 3), cy = __ldcs(coords + i * 3 + 1), cx = __ldcs(coords + i * 3 + 2);
+        if (inside3(cz, cy, cx, g.D, g.H, g.W)) {
+            c[0] = cz;
+            c[1] = cy;
+            c[2] = cx;
+            if constexpr (E == 2) {
+                const float2 v = __ldcs(vals + i);
+                re = v.x;
+                im = v.y;
+            } else {
+                re = __ldcs(vals + i);
+            }
+        }
+    }
+    insert_point_octet(acc, g, re, im, 1.0f, c, tab[threadIdx.x >> 5], false);  // every lane takes part
+}
+
+// image += values, weights += weights of the bricked accumulator; one warp per
+// brick row.
+template <int E>
+__global__ void __launch_bounds__(256)
+splat_finish_kernel(const float4* __restrict__ acc, typename Vec<E>::T* __restrict__ img, float* __restrict__ wts,
+                    SliceGeom g) {
+    const int bh = (g.H + 1) >> 1, bw = (g.W + 1) >> 1;
+    const int64_t rowi = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int bz = (int)(rowi / bh), by = (int)(rowi - (int64_t)bz * bh);
+    if (2 * bz >= g.D) return;
+    const float4* row = acc + rowi * bw * 8;
+    for (int t = threadIdx.x & 31; t < bw * 8; t += 32) {
+        const int z = 2 * bz + ((t >> 2) & 1), y = 2 * by + ((t >> 1) & 1), x = 2 * (t >> 3) + (t & 1);
+        if (z >= g.D || y >= g.H || x >= g.W) continue;
+        const float4 a = __ldcs(row + t);
+        if (a.x == 0.0f && a.y == 0.0f && a.z == 0.0f) continue;
+        const int64_t o = ((int64_t)z * g.H + y) * g.W + x;
+        if constexpr (E == 2) {
+            const float2 v = img[o];
+            img[o] = make_float2(v.x + a.x, v.y + a.y);
+        } else {
+            img[o] += a.x;
+        }
+        wts[o] += a.z;
+    }
+}
+
 inline unsigned nblocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 // The single-precision trilinear kernels take up to 4096 channels; 8-byte
@@ -474,6 +532,18 @@ inline bool f32_path(int32_t dtype, int32_t nearest, int64_t channels, const voi
     const uintptr_t mask = dtype == 2 ? 7 : 3;
     return (dtype == 0 || dtype == 2) && !nearest && channels <= 4096 &&
            (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & mask) == 0;
+}
+
+// Bytes of the bricked accumulator, or 0 where the direct splat is used: the
+// accumulator's zeroing and the last pass cost about 12 ps a voxel, the splat
+// 22 ps a point against 39 (measured at 192^3 / 2, 9.3 M points: 256 against 361
+// us), so from one point per voxel.
+inline size_t splat_bytes(int32_t dtype, int64_t n, int64_t channels, int64_t d, int64_t h, int64_t w,
+                          int32_t weights_f64, int32_t nearest) {
+    if ((dtype != 0 && dtype != 2) || nearest || weights_f64 || channels != 1 || d < 1 || h < 1 || w < 1) return 0;
+    if (d > (1 << 20) || h > (1 << 20) || w > (1 << 20)) return 0;
+    const int64_t slots = ((d + 1) / 2) * ((h + 1) / 2) * ((w + 1) / 2) * 8;
+    return n >= 200000 && n >= d * h * w && slots < (1LL << 31) ? (size_t)slots * sizeof(float4) : 0;
 }
 inline bool idx32(int64_t channels, int64_t d, int64_t h, int64_t w) { return channels * d * h * w < (1LL << 31); }
 
@@ -571,6 +641,45 @@ extern "C" int tt_insert_into_image_3d(const void* values, int32_t dtype, const 
     }
 #undef TT_INSERT_CASE
     return check_launch("insert3d_kernel");
+}
+
+extern "C" size_t tt_insert_into_image_3d_workspace_bytes(int32_t dtype, int64_t n, int64_t channels, int64_t d,
+                                                          int64_t h, int64_t w, int32_t weights_f64,
+                                                          int32_t nearest) {
+    return splat_bytes(dtype, n, channels, d, h, w, weights_f64, nearest);
+}
+
+extern "C" int tt_insert_into_image_3d_workspace(const void* values, int32_t dtype, const float* coordinates,
+                                                 int64_t n, void* image, int64_t channels, int64_t d, int64_t h,
+                                                 int64_t w, void* weights, int32_t weights_f64, int32_t nearest,
+                                                 void* workspace, size_t workspace_bytes, void* stream) {
+    const size_t need = splat_bytes(dtype, n, channels, d, h, w, weights_f64, nearest);
+    if (!need || !f32_path(dtype, nearest, channels, values, image, nullptr))
+        return tt_insert_into_image_3d(values, dtype, coordinates, n, image, channels, d, h, w, weights, weights_f64,
+                                       nearest, stream);
+    if (!values || !coordinates || !image || !weights)
+        return fail(TT_ERR_INVALID, "insert_into_image_3d: bad arguments");
+    if (!workspace || workspace_bytes < need)
+        return fail(TT_ERR_WORKSPACE, "insert_into_image_3d: workspace of %zu bytes needed, got %zu", need,
+                    workspace_bytes);
+    if ((n + 255) / 256 > 0x7fffffffLL) return fail(TT_ERR_INVALID, "insert_into_image_3d: too many points");
+    cudaStream_t st = as_stream(stream);
+    cudaError_t e = cudaMemsetAsync(workspace, 0, need, st);
+    if (e != cudaSuccess) return fail(TT_ERR_CUDA, "insert_into_image_3d: memset: %s", cudaGetErrorString(e));
+    SliceGeom g{};  // the splat and its last pass read the image dims only
+    g.D = (int)d;
+    g.H = (int)h;
+    g.W = (int)w;
+    float4* acc = (float4*)workspace;
+    const unsigned rows = nblocks(((d + 1) / 2) * ((h + 1) / 2), 8);
+    if (dtype == 2) {
+        splat_bricked_kernel<2><<<nblocks(n, 256), 256, 0, st>>>((const float2*)values, coordinates, n, acc, g);
+        splat_finish_kernel<2><<<rows, 256, 0, st>>>(acc, (float2*)image, (float*)weights, g);
+    } else {
+        splat_bricked_kernel<1><<<nblocks(n, 256), 256, 0, st>>>((const float*)values, coordinates, n, acc, g);
+        splat_finish_kernel<1><<<rows, 256, 0, st>>>(acc, (float*)image, (float*)weights, g);
+    }
+    return check_launch("splat_bricked_kernel");
 }
 
 extern "C" int tt_affine_transform_image_3d(const void* image, int32_t dtype, int64_t channels, int64_t d, int64_t h,

@@ -134,10 +134,13 @@ class _InsertIntoImage3d(torch.autograd.Function):
         d, h, w = image.shape[-3:]
         v = _lib.dense(vals)
         L = _lib.load()
-        _lib.check(L.tt_insert_into_image_3d(_lib.ptr(v), _code(image.dtype), _lib.ptr(coords), coords.shape[0],
-                                             _lib.ptr(image), C, d, h, w, _lib.ptr(weights),
-                                             int(weights.dtype == torch.float64), int(nearest),
-                                             _lib.stream_of(image.device)), "insert_into_image_3d")
+        n, wide = coords.shape[0], int(weights.dtype == torch.float64)
+        nbytes = int(L.tt_insert_into_image_3d_workspace_bytes(_code(image.dtype), n, C, d, h, w, wide, int(nearest)))
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=image.device) if nbytes else None
+        _lib.check(L.tt_insert_into_image_3d_workspace(_lib.ptr(v), _code(image.dtype), _lib.ptr(coords), n,
+                                                       _lib.ptr(image), C, d, h, w, _lib.ptr(weights), wide,
+                                                       int(nearest), _lib.ptr(ws), nbytes,
+                                                       _lib.stream_of(image.device)), "insert_into_image_3d")
         ctx.mark_dirty(image, weights)
         ctx.mark_non_differentiable(weights)
         ctx.save_for_backward(coords)

@@ -86,6 +86,28 @@ def test_insert(shape, c, n, dtype, wdtype):
     assert torch.equal(wts[same], wstart.to(wdtype)[same]) and torch.equal(img[:, same], start[:, same])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.complex64])
+@pytest.mark.parametrize("shape,n", [((24, 31, 17), 200003), ((1, 300, 5), 200000), ((58, 58, 59), 200000),
+                                     ((60, 60, 60), 210000)])
+def test_insert_many_points(shape, n, dtype):
+    """From one point per voxel (and 200,000 points) the splat goes through a
+    bricked accumulator; the third shape has 198,476 voxels, just enough, the
+    last 216,000, too many.  Neighbouring points in neighbouring, equal and far
+    cells."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    co = _points(n, shape, g)
+    step = torch.tensor([0.3, 0.5, 0.8], device="cuda")
+    k = torch.arange(n // 2, device="cuda") % 32
+    co[: n // 2] = co[: n // 2 : 32].repeat_interleave(32, 0)[: n // 2] + k[:, None] * step  # runs of points
+    vals = _randn((n,), dtype, g)
+    start, wstart = _randn(shape, dtype, g), torch.rand(shape, generator=g, device="cuda")
+    img, wts = tt().insert_into_image_3d(vals, co, start.clone(), wstart.clone())
+    ref, rw = tt().insert_into_image_3d(vals.to(WIDE[dtype]), co, start.to(WIDE[dtype]), wstart.double())
+    assert rel_l2(img.cpu().numpy(), ref.cpu().numpy()) < 3e-6 and rel_l2(wts.cpu().numpy(), rw.cpu().numpy()) < 3e-6
+    same = rw == wstart.double()
+    assert torch.equal(wts[same], wstart[same]) and torch.equal(img[same], start[same])
+
+
 def test_non_finite_values():
     """Infinities and NaN in the image reach the same samples, and those in the upstream
     gradient the same voxels, as in double precision."""
