@@ -34,13 +34,12 @@ constexpr int kExtractThreads = kTileThreads;
 
 // Parts a row of tiles is split into so that `blocks` rows fill the chip: with
 // fewer than two waves of resident blocks a row's tiles run one after the
-// other in a few blocks while the other SMs idle.  Up to four waves, at least
-// `least` tiles a part.  8 slices of 96: 8.6 -> 3.6 us; 100 slices of 128: 16 ->
+// other in a few blocks while the other SMs idle, and with few waves the last
+// one is nearly empty.  Up to six waves, at least `least` tiles a part.  8 slices of 96: 8.6 -> 3.6 us; 100 slices of 128: 16 ->
 // 10 us.
 static int row_splits(int64_t blocks, int tx_tiles, int resident, int least) {
-    const int64_t wave = 148 * resident;
-    if (blocks >= 4 * wave) return 1;
-    const int64_t want = (4 * wave + blocks - 1) / blocks, most = tx_tiles / least;
+    const int64_t fill = 6 * 148 * resident;
+    const int64_t want = blocks < 1 ? 1 : (fill + blocks - 1) / blocks, most = tx_tiles / least;
     const int64_t k = want < most ? want : most;
     return (int)(k < 1 ? 1 : k);
 }
@@ -205,7 +204,8 @@ __device__ __forceinline__ void mse_point(const VT* __restrict__ vol, const floa
 // rotation-gradient partials reduced once per row.  WANT_DR: the row's sums of
 // the 6 non-zero entries of d/dR_zyx (per thread over its pixels, warp totals
 // in float, then the eight warps in double, in a fixed order) go to
-// part[(s * rows + row) * 6 + k], one slot per row of tiles.  FIXED:
+// part[((s * rows + row) * parts + part) * 6 + k], one slot per part of a row
+// (gridDim.y parts: row_splits).  FIXED:
 // the volume gradient goes to the
 // fixed-point words `fixed` at the scale set by *absmax and n.  Resident
 // blocks: 6 for the rotation gradient alone (39 registers), 5 with the volume
@@ -227,7 +227,9 @@ extract_bwd_kernel(const VT* __restrict__ vol, const void* __restrict__ rot,
     float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     DvTarget<FIXED> dv{dvol, fixed, 0.0};
     if (FIXED) dv.scale = fixed_data_scale(*absmax, ceil_log2(g.n));
-    for (int tx = 0; tx < tx_tiles; tx++) {  // every lane runs every tile (the paired scatter shuffles)
+    const int last = split_tile(tx_tiles, blockIdx.y + 1);
+    // every lane runs every tile (the paired scatter shuffles)
+    for (int tx = split_tile(tx_tiles, blockIdx.y); tx < last; tx++) {
         int iy, ix;
         const bool has_pixel = tile_pixel(g, ty * tx_tiles + tx, iy, ix);
         bwd_point<WANT_DV, WANT_DR, FIXED, VT>(vol, m, grad, dv, g, s, has_pixel, iy, ix, acc);
@@ -243,7 +245,7 @@ extract_bwd_kernel(const VT* __restrict__ vol, const void* __restrict__ rot,
             double v = 0.0;
 #pragma unroll
             for (int w = 0; w < kExtractThreads / 32; w++) v += red[w][threadIdx.x];
-            part[((int64_t)s * rows + ty) * 6 + threadIdx.x] = (float)v;
+            part[(((int64_t)s * rows + ty) * gridDim.y + blockIdx.y) * 6 + threadIdx.x] = (float)v;
         }
     }
 }
@@ -251,7 +253,7 @@ extract_bwd_kernel(const VT* __restrict__ vol, const void* __restrict__ rot,
 // Fused extraction + mean squared error + backward: one block per (slice, row
 // of tiles).  The row's partials of the loss (double) go to
 // loss_part[s * rows + row] and, with WANT_DR, those of d/dR_zyx to
-// part[(s * rows + row) * 6 + k]: one slot per row of tiles.
+// part[.. * 6 + k]: one slot per part of a row of tiles, as in the backward.
 // Five resident blocks (48 registers); four for the rotation gradient alone,
 // which spills at 48 (256^3 x 4096: 1.95 vs 2.19 ms at five).
 template <bool WANT_DV, bool WANT_DR, typename VT>
@@ -270,7 +272,9 @@ slice_mse_kernel(const VT* __restrict__ vol, const void* __restrict__ rot, const
     float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     double loss = 0.0;
     const DvTarget<false> dv{dvol, nullptr, 0.0};
-    for (int tx = 0; tx < tx_tiles; tx++) {  // every lane runs every tile (the paired scatter shuffles)
+    const int last = split_tile(tx_tiles, blockIdx.y + 1);
+    // every lane runs every tile (the paired scatter shuffles)
+    for (int tx = split_tile(tx_tiles, blockIdx.y); tx < last; tx++) {
         int iy, ix;
         const bool has_pixel = tile_pixel(g, ty * tx_tiles + tx, iy, ix);
         mse_point<WANT_DV, WANT_DR, VT>(vol, m, target, dv, g, s, has_pixel, iy, ix, scale, acc, loss);
@@ -287,7 +291,7 @@ slice_mse_kernel(const VT* __restrict__ vol, const void* __restrict__ rot, const
         double v = 0.0;
 #pragma unroll
         for (int w = 0; w < kExtractThreads / 32; w++) v += red[w][threadIdx.x];
-        const int64_t b0 = (int64_t)s * rows + ty;
+        const int64_t b0 = ((int64_t)s * rows + ty) * gridDim.y + blockIdx.y;
         if (threadIdx.x == 6)
             loss_part[b0] = v;
         else if (WANT_DR)
@@ -393,8 +397,11 @@ __global__ void dv_fixed_add_kernel(const long long* __restrict__ fixed, float2*
 // multichannel ones).
 static size_t partial_bytes(int64_t n, int parts) { return (size_t)(n * parts * 6) * sizeof(float); }
 
-// Rows of tiles per slice: the single-channel kernels' blocks and partial slots.
+// Rows of tiles per slice, and the parts a row is split into by the backward
+// and the fused loss: their blocks and partial slots.  256 slices of 180, both
+// gradients: 124 -> 115 us.
 static int tile_rows(int img_h) { return (img_h + kTileY - 1) / kTileY; }
+static int grad_splits(int64_t n, int img_h, int wr) { return row_splits(n * tile_rows(img_h), tiles_x_of(wr), 5, 4); }
 
 int launch_drot_finish(const float* part, const void* rot, void* drot, const SliceGeom& g, int parts,
                        cudaStream_t st) {
@@ -416,7 +423,9 @@ template <typename VT>
 static int launch_backward_t(const VT* v, const void* rot, const float2* gr, float2* dv, void* grad_rotation,
                              float* part, const SliceGeom& g, cudaStream_t st, void* fixed) {
     const int tiles = extract_tiles(g);
-    const unsigned blocks = (unsigned)((int64_t)g.n * (tiles / tiles_x_of(g.wr)));  // one block per row of tiles
+    // one block per row of tiles, or per part of one
+    const int splits = grad_splits(g.n, g.img_h, g.wr);
+    const dim3 blocks((unsigned)((int64_t)g.n * tile_rows(g.img_h)), (unsigned)splits);
     uint32_t* absmax = (uint32_t*)fixed;
     unsigned long long* facc = fixed ? (unsigned long long*)((char*)fixed + kFixedHeaderBytes) : nullptr;
     if (dv && fixed) {
@@ -443,7 +452,7 @@ static int launch_backward_t(const VT* v, const void* rot, const float2* gr, flo
     }
     if (int e = check_launch("extract_bwd_kernel")) return e;
     if (grad_rotation)
-        if (int e = launch_drot_finish(part, rot, grad_rotation, g, tile_rows(g.img_h), st)) return e;
+        if (int e = launch_drot_finish(part, rot, grad_rotation, g, tile_rows(g.img_h) * splits, st)) return e;
     return TT_OK;
 }
 
@@ -516,7 +525,7 @@ __global__ void pack_xpairs_kernel(const float2* __restrict__ vol, float4* __res
 
 template <typename VT>
 static int launch_mse(const VT* v, const void* rot, const float2* t, float2* dv, void* grad_rotation, float* part,
-                      double* loss_part, float scale, const SliceGeom& g, int tiles, unsigned nb, cudaStream_t st) {
+                      double* loss_part, float scale, const SliceGeom& g, int tiles, dim3 nb, cudaStream_t st) {
     if (dv && grad_rotation)
         slice_mse_kernel<true, true, VT><<<nb, kExtractThreads, 0, st>>>(v, rot, t, dv, part, loss_part, scale, g,
                                                                         tiles);
@@ -536,14 +545,15 @@ static int launch_mse(const VT* v, const void* rot, const float2* t, float2* dv,
 
 using namespace tt;
 
-// Loss partials (double) and rotation-gradient partials, one slot per row of tiles.
-static size_t mse_workspace_bytes(int64_t n, int rows) {
-    return (size_t)(n * rows) * sizeof(double) + partial_bytes(n, rows);
+// Loss partials (double) and rotation-gradient partials, `parts` slots per slice.
+static size_t mse_workspace_bytes(int64_t n, int parts) {
+    return (size_t)(n * parts) * sizeof(double) + partial_bytes(n, parts);
 }
+static int mse_parts(int64_t n, int img_h, int wr) { return tile_rows(img_h) * grad_splits(n, img_h, wr); }
 
 extern "C" size_t tt_central_slice_mse_workspace_bytes(const tt_slice_params* p) {
     if (!p || p->n <= 0 || p->img_h < 1 || p->img_w < 1) return 0;
-    return mse_workspace_bytes(p->n, tile_rows((int)p->img_h));
+    return mse_workspace_bytes(p->n, mse_parts(p->n, (int)p->img_h, (int)(p->img_w / 2 + 1)));
 }
 
 extern "C" int tt_central_slice_mse(const void* volume_rfft, const void* rotation_matrices, const void* targets,
@@ -558,10 +568,10 @@ extern "C" int tt_central_slice_mse(const void* volume_rfft, const void* rotatio
         return fail(TT_ERR_INVALID, "central_slice_mse: NULL pointer argument");
     SliceGeom g = make_geom(*p);
     const int tiles = extract_tiles(g);
-    const int rows = tile_rows(g.img_h);
-    const int64_t blocks = (int64_t)g.n * rows;  // one block (and one partial slot) per row of tiles
+    const int parts = mse_parts(g.n, g.img_h, g.wr);
+    const int64_t blocks = (int64_t)g.n * parts;  // one block and one partial slot per part of a row of tiles
     if ((int64_t)g.n * tiles > 0x7fffffffLL) return fail(TT_ERR_INVALID, "central_slice_mse: too many blocks");
-    const size_t need = mse_workspace_bytes(g.n, rows);
+    const size_t need = mse_workspace_bytes(g.n, parts);
     if (!workspace || workspace_bytes < need)
         return fail(TT_ERR_WORKSPACE, "central_slice_mse: workspace of %zu bytes needed, got %zu", need,
                     workspace_bytes);
@@ -572,7 +582,8 @@ extern "C" int tt_central_slice_mse(const void* volume_rfft, const void* rotatio
     const float2* t = (const float2*)targets;
     float2* dv = (float2*)grad_volume;
     cudaStream_t st = as_stream(stream);
-    const unsigned nb = (unsigned)((int64_t)g.n * (tiles / tiles_x_of(g.wr)));  // one block per row of tiles
+    const int rows = tile_rows(g.img_h);
+    const dim3 nb((unsigned)((int64_t)g.n * rows), (unsigned)(parts / rows));
     int e;
     switch (g.vol_layout) {
         case TT_VOLUME_XPAIRS:
@@ -590,7 +601,7 @@ extern "C" int tt_central_slice_mse(const void* volume_rfft, const void* rotatio
     if (e) return e;
     mse_loss_finish_kernel<<<1, 1024, 0, st>>>(loss_part, blocks, 1.0 / m, loss);
     if (int e = check_launch("mse_loss_finish_kernel")) return e;
-    if (grad_rotation) return launch_drot_finish(part, rotation_matrices, grad_rotation, g, rows, st);
+    if (grad_rotation) return launch_drot_finish(part, rotation_matrices, grad_rotation, g, parts, st);
     return TT_OK;
 }
 
@@ -696,7 +707,8 @@ extern "C" int tt_extract_central_slices_rfft_3d_backward(
     if ((int64_t)g.n * tiles > 0x7fffffffLL) return fail(TT_ERR_INVALID, "extract backward: too many blocks");
     const size_t fixed = grad_volume ? fixed_dv_bytes(p) : 0;
     if (grad_rotation || fixed) {
-        const size_t need = fixed + (grad_rotation ? partial_bytes(g.n, tile_rows(g.img_h)) : 0);
+        const size_t need =
+            fixed + (grad_rotation ? partial_bytes(g.n, tile_rows(g.img_h) * grad_splits(g.n, g.img_h, g.wr)) : 0);
         if (!workspace || workspace_bytes < need)
             return fail(TT_ERR_WORKSPACE, "extract backward: workspace of %zu bytes needed, got %zu", need,
                         workspace_bytes);
@@ -779,10 +791,11 @@ extern "C" int tt_extract_central_slices_rfft_3d_backward_noalloc(const void* vo
     const void* v = volume_rfft;
     const float2* gr = (const float2*)grad_slices;
     float2* dv = (float2*)grad_volume;
-    // the scratch holds 6 partial sums of the rotation gradient per row of tiles
+    // the scratch holds 6 partial sums of the rotation gradient per row of tiles (per
+    // part of a row where the launch is small: far from the array's limit)
     if (!grad_rotation)  // the volume gradient alone needs no scratch
         return launch_backward(v, rotation_matrices, gr, dv, nullptr, nullptr, g, st);
-    const size_t need = partial_bytes(g.n, tile_rows(g.img_h));
+    const size_t need = partial_bytes(g.n, tile_rows(g.img_h) * grad_splits(g.n, g.img_h, g.wr));
     if (need > (size_t)TT_NOALLOC_SCRATCH_BYTES)
         return fail(TT_ERR_INVALID,
                     "noalloc backward: %lld slices of %lld x %lld need %zu bytes of scratch, more than the "
