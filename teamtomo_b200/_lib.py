@@ -177,20 +177,38 @@ def dense(t: torch.Tensor) -> torch.Tensor:
     """``t`` as a C-contiguous tensor whose memory holds its values: lazy
     conjugate / negative views (``x.conj()``, and the gradients autograd
     passes through them) are materialised first."""
+    if t.is_contiguous() and not t.is_conj() and not t.is_neg():
+        return t
     return t.resolve_conj().resolve_neg().contiguous()
 
 
-def ptr(t: torch.Tensor | None):
+def ptr(t: torch.Tensor | None) -> int | None:
+    """Address of ``t``'s memory, as the C entry points' pointer arguments take it."""
     if t is None:
         return None
     if t.is_conj() or t.is_neg():
         # the memory of a lazy view does not hold its values
         raise ValueError("tensor is a lazy conjugate/negative view; materialise it with dense()")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
-def stream_of(device: torch.device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def stream_of(device: torch.device) -> int:
+    """Handle of the device's current stream (without a torch.cuda.Stream object)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+def untracked(*tensors: torch.Tensor) -> bool:
+    """Whether no derivative of a call on ``tensors`` can be asked for: no
+    backward (grad mode off or nothing requires grad), no forward-mode level and
+    no functorch transform (vmap, jvp, ..).  ``Function.apply`` then does nothing
+    but run the forward, which such calls do directly (its bookkeeping takes
+    about a third of a small call's host time)."""
+    if torch.is_grad_enabled():
+        for t in tensors:
+            if t.requires_grad:
+                return False
+    return torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
 
 
 def require_cuda(*tensors: torch.Tensor) -> torch.device:

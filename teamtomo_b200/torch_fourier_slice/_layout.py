@@ -46,7 +46,8 @@ MIN_PIXELS_PER_VOXEL = 0.5
 
 
 def _mode() -> str:
-    return os.environ.get("TT_VOLUME_LAYOUT", "auto").strip().lower()
+    mode = os.environ.get("TT_VOLUME_LAYOUT", "auto")
+    return mode if mode == "auto" else mode.strip().lower()
 
 
 def automatic() -> bool:
@@ -79,7 +80,10 @@ def bricks_fit(volume: torch.Tensor) -> bool:
 
 
 def with_layout(params: _lib.SliceParams, layout: int) -> _lib.SliceParams:
-    """Copy of ``params`` with ``volume_layout`` set to ``layout``."""
+    """Copy of ``params`` with ``volume_layout`` set to ``layout`` (``params``
+    itself where it has that layout)."""
+    if params.volume_layout == int(layout):
+        return params
     q = _lib.SliceParams()
     ctypes.pointer(q)[0] = params
     q.volume_layout = int(layout)

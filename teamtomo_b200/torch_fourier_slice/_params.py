@@ -2,6 +2,8 @@
 
 from __future__ import annotations
 
+from functools import lru_cache
+
 import numpy as np
 import torch
 
@@ -20,35 +22,34 @@ def rotation_arg(rotation_matrices: torch.Tensor, device: torch.device):
     stack = tuple(R.shape[:-2])
     if R.dtype not in (torch.float32, torch.float64):
         R = R.to(torch.float32)
-    R = R.to(device).reshape(-1, 3, 3).contiguous()
-    return R, stack
+    if R.device != device:
+        R = R.to(device)
+    if R.ndim != 3:
+        R = R.reshape(-1, 3, 3)
+    return R.contiguous(), stack
 
 
-def _f32(x: float) -> float:
+@lru_cache(maxsize=256)
+def _rounded(x: float) -> float:
     return float(np.float32(x))
+
+
+def _f32(x) -> float:
+    return _rounded(float(x))
 
 
 def slice_params(n, image_shape, volume, rotation, fftfreq_max=None, zyx_matrices=False,
                  x_tolerance=1e-8, rot_tolerance=None, volume_unshifted=False,
                  slices_unshifted=False, vol_dims=None, deterministic=False) -> _lib.SliceParams:
     d, h, w = (int(s) for s in image_shape)
-    vd, vh, vw = vol_dims if vol_dims is not None else tuple(int(s) for s in volume.shape[-3:])
-    p = _lib.SliceParams()
-    p.n = int(n)
-    p.img_d, p.img_h, p.img_w = d, h, w
-    p.vol_d, p.vol_h, p.vol_w = vd, vh, vw
-    p.has_fftfreq_max = int(fftfreq_max is not None)
-    p.fftfreq_max = _f32(fftfreq_max) if fftfreq_max is not None else 0.0
-    p.zyx_matrices = int(bool(zyx_matrices))
-    p.x_tolerance = _f32(x_tolerance)
-    p.x_tolerance10 = _f32(x_tolerance * 10)
-    p.has_rot_tolerance = int(rot_tolerance is not None)
-    p.rot_tolerance = _f32(rot_tolerance) if rot_tolerance is not None else 0.0
-    p.rotation_f64 = int(rotation.dtype == torch.float64)
-    p.volume_unshifted = int(bool(volume_unshifted))
-    p.slices_unshifted = int(bool(slices_unshifted))
-    p.deterministic = int(bool(deterministic))
-    return p
+    vd, vh, vw = vol_dims if vol_dims is not None else (int(s) for s in volume.shape[-3:])
+    return _lib.SliceParams(
+        int(n), d, h, w, vd, vh, vw,
+        int(fftfreq_max is not None), _f32(fftfreq_max) if fftfreq_max is not None else 0.0,
+        int(bool(zyx_matrices)), _f32(x_tolerance), _f32(x_tolerance * 10),
+        int(rot_tolerance is not None), _f32(rot_tolerance) if rot_tolerance is not None else 0.0,
+        int(rotation.dtype == torch.float64), int(bool(volume_unshifted)), int(bool(slices_unshifted)),
+        int(bool(deterministic)), 0)
 
 
 def resolve_deterministic(flag: bool | None) -> bool:

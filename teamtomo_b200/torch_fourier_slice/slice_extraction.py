@@ -27,26 +27,32 @@ from . import _layout
 from ._params import resolve_deterministic, rotation_arg, slice_params
 
 
+def _extract(volume_rfft, rotation_matrices, params, out_shape):
+    """(slices, volume copy the gathers read or None, its layout)."""
+    # the kernels index raw memory in C order and sample complex64
+    if not (volume_rfft.is_contiguous() and rotation_matrices.is_contiguous()):
+        raise ValueError("extraction needs C-contiguous volume and rotation tensors")
+    if volume_rfft.dtype != torch.complex64:
+        raise RuntimeError(f"the extraction kernels sample complex64 volumes (got {volume_rfft.dtype})")
+    dev = volume_rfft.device
+    out = torch.empty(out_shape, dtype=torch.complex64, device=dev)
+    L = _lib.load()
+    # large calls gather from a bricked copy (bit-identical results)
+    layout = _layout.choose(out.numel(), volume_rfft)
+    copy = _layout.pack(volume_rfft, params, layout)
+    _lib.check(
+        L.tt_extract_central_slices_rfft_3d(_lib.ptr(copy if copy is not None else volume_rfft),
+                                            _lib.ptr(rotation_matrices), _lib.ptr(out),
+                                            _layout.with_layout(params, layout), _lib.stream_of(dev)),
+        "extract_central_slices_rfft_3d",
+    )
+    return out, copy, layout
+
+
 class _ExtractCentralSlices(torch.autograd.Function):
     @staticmethod
     def forward(ctx, volume_rfft, rotation_matrices, params, out_shape):
-        # the kernels index raw memory in C order and sample complex64
-        if not (volume_rfft.is_contiguous() and rotation_matrices.is_contiguous()):
-            raise ValueError("extraction needs C-contiguous volume and rotation tensors")
-        if volume_rfft.dtype != torch.complex64:
-            raise RuntimeError(f"the extraction kernels sample complex64 volumes (got {volume_rfft.dtype})")
-        dev = volume_rfft.device
-        out = torch.empty(out_shape, dtype=torch.complex64, device=dev)
-        L = _lib.load()
-        # large calls gather from a bricked copy (bit-identical results)
-        layout = _layout.choose(out.numel(), volume_rfft)
-        copy = _layout.pack(volume_rfft, params, layout)
-        _lib.check(
-            L.tt_extract_central_slices_rfft_3d(_lib.ptr(copy if copy is not None else volume_rfft),
-                                                _lib.ptr(rotation_matrices), _lib.ptr(out),
-                                                _layout.with_layout(params, layout), _lib.stream_of(dev)),
-            "extract_central_slices_rfft_3d",
-        )
+        out, copy, layout = _extract(volume_rfft, rotation_matrices, params, out_shape)
         ctx.params = params
         # the backward reads the volume only for d/drotation: keep the copy for it
         keep = copy is not None and ctx.needs_input_grad[1]
@@ -194,8 +200,12 @@ def extract_central_slices_rfft_3d(
                           rotation=R, fftfreq_max=fftfreq_max, zyx_matrices=zyx_matrices,
                           x_tolerance=x_tolerance, rot_tolerance=rot_tolerance,
                           deterministic=resolve_deterministic(deterministic))
-    out = _ExtractCentralSlices.apply(volume_rfft, R, params, (R.shape[0], h, w // 2 + 1))
-    return out.reshape(*stack, h, w // 2 + 1)
+    shape = (R.shape[0], h, w // 2 + 1)
+    if _lib.untracked(volume_rfft, R):
+        out = _extract(volume_rfft, R, params, shape)[0]
+    else:
+        out = _ExtractCentralSlices.apply(volume_rfft, R, params, shape)
+    return out if len(stack) == 1 else out.reshape(*stack, h, w // 2 + 1)
 
 
 def central_slice_geometry(

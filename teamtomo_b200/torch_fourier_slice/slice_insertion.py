@@ -256,6 +256,19 @@ def insert_backward_multichannel(grad_volumes, R, volume_shape, fftfreq_max=None
     return out
 
 
+def _insert(images, R, volume_shape, fftfreq_max, zyx_matrices, deterministic, unshifted=False):
+    """(n, c, h, w//2+1) slices -> ((c, d, h, w//2+1) volumes, weights)."""
+    c = images.shape[1]
+    c128 = images.dtype == torch.complex128
+    if c > 1 and not c128 and not deterministic:
+        # one geometry pass per pixel for all channels
+        acc = new_accumulator(volume_shape, False, images.device, channels=c)
+        insert_accumulate_multichannel(_lib.dense(images), R, volume_shape, acc, fftfreq_max, zyx_matrices, unshifted)
+        return insert_finalize(acc, False)
+    chans = [_lib.dense(images[:, ch]) for ch in range(c)]
+    return _splat(chans, R, volume_shape, fftfreq_max, zyx_matrices, deterministic, c128, images.device, unshifted)
+
+
 class _InsertCentralSlices(torch.autograd.Function):
     """(n, c, h, w//2+1) slices -> ((c, d, h, w//2+1) volumes, weights),
     differentiable w.r.t. the slices (not the rotations, which are constants
@@ -264,18 +277,7 @@ class _InsertCentralSlices(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, images, R, volume_shape, fftfreq_max, zyx_matrices, deterministic, unshifted=False):
-        c = images.shape[1]
-        c128 = images.dtype == torch.complex128
-        if c > 1 and not c128 and not deterministic:
-            # one geometry pass per pixel for all channels
-            acc = new_accumulator(volume_shape, False, images.device, channels=c)
-            insert_accumulate_multichannel(_lib.dense(images), R, volume_shape, acc, fftfreq_max, zyx_matrices,
-                                           unshifted)
-            volumes, weights = insert_finalize(acc, False)
-        else:
-            chans = [_lib.dense(images[:, ch]) for ch in range(c)]
-            volumes, weights = _splat(chans, R, volume_shape, fftfreq_max, zyx_matrices, deterministic, c128,
-                                      images.device, unshifted)
+        volumes, weights = _insert(images, R, volume_shape, fftfreq_max, zyx_matrices, deterministic, unshifted)
         ctx.mark_non_differentiable(weights)
         ctx.save_for_backward(R)
         ctx.args = (volume_shape, fftfreq_max, zyx_matrices, unshifted)
@@ -315,8 +317,9 @@ def insert_central_slices_rfft_3d(
     if math.prod(lead) != n:
         raise ValueError(f"{n} rotation matrices for image stack of shape {tuple(lead)}")
     img = image_rfft.reshape(n, 1, *image_rfft.shape[-2:])
-    volumes, weights = _InsertCentralSlices.apply(img, R, tuple(int(x) for x in volume_shape), fftfreq_max,
-                                                  zyx_matrices, resolve_deterministic(deterministic))
+    args = (img, R, tuple(int(x) for x in volume_shape), fftfreq_max, zyx_matrices,
+            resolve_deterministic(deterministic))
+    volumes, weights = _insert(*args) if _lib.untracked(img, R) else _InsertCentralSlices.apply(*args)
     return volumes[0], weights
 
 
@@ -338,5 +341,6 @@ def insert_central_slices_rfft_3d_multichannel(
     R, stack = rotation_arg(rotation_matrices, dev)
     n = R.shape[0]
     img = image_rfft.reshape(n, c, *image_rfft.shape[-2:])
-    return _InsertCentralSlices.apply(img, R, tuple(int(x) for x in volume_shape), fftfreq_max, zyx_matrices,
-                                      resolve_deterministic(deterministic))
+    args = (img, R, tuple(int(x) for x in volume_shape), fftfreq_max, zyx_matrices,
+            resolve_deterministic(deterministic))
+    return _insert(*args) if _lib.untracked(img, R) else _InsertCentralSlices.apply(*args)

@@ -27,18 +27,22 @@ def _code(dtype: torch.dtype) -> int:
     return _DTYPE_CODES[dtype]
 
 
+def _sample(img, coords, nearest):
+    C, D, H, W = img.shape
+    n = coords.shape[0]
+    out = torch.empty((n, C), dtype=img.dtype, device=img.device)
+    L = _lib.load()
+    _lib.check(L.tt_sample_image_3d(_lib.ptr(img), _code(img.dtype), C, D, H, W, _lib.ptr(coords), n,
+                                    _lib.ptr(out), int(nearest), _lib.stream_of(img.device)), "sample_image_3d")
+    return out
+
+
 class _SampleImage3d(torch.autograd.Function):
     @staticmethod
     def forward(ctx, img, coords, nearest):
-        C, D, H, W = img.shape
-        n = coords.shape[0]
-        out = torch.empty((n, C), dtype=img.dtype, device=img.device)
-        L = _lib.load()
-        _lib.check(L.tt_sample_image_3d(_lib.ptr(img), _code(img.dtype), C, D, H, W, _lib.ptr(coords), n,
-                                        _lib.ptr(out), int(nearest), _lib.stream_of(img.device)), "sample_image_3d")
         ctx.save_for_backward(img, coords)
         ctx.nearest = nearest
-        return out
+        return _sample(img, coords, nearest)
 
     @staticmethod
     def backward(ctx, grad):
@@ -79,7 +83,8 @@ def sample_image_3d(
     coords = torch.as_tensor(coordinates).to(image.device)
     batch = coords.shape[:-1]
     c = _lib.dense(coords.reshape(-1, 3).to(_REAL[image.dtype]))
-    out = _SampleImage3d.apply(img, c, interpolation == "nearest")
+    sample = _sample if _lib.untracked(img, c) else _SampleImage3d.apply
+    out = sample(img, c, interpolation == "nearest")
     return out.reshape(*batch, C) if multi else out.reshape(batch)
 
 
