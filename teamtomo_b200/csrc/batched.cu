@@ -126,20 +126,21 @@ batched_slices_kernel(const __grid_constant__ BatchParams bp, unsigned long long
                 }
             }
         } else {
-            for (int tx = 0; tx < txt; tx++) {
-                // z-phased filling of large accumulators (the same answer in every thread)
-                if (nphase > 1 && insert_tile_phase(bv.g, m, min(ty * TY + TY / 2, bv.g.img_h - 1),
-                                                    min(tx * TX + TX / 2, bv.g.wr - 1), nphase) != phase)
-                    continue;
-                const int ix = tx * TX + (lane % TX);
-                const bool has_pixel = ix < bv.g.wr && iy < bv.g.img_h;
-                // every lane takes part: lane octets (bricked accumulator) or lane pairs share a pixel
-                if (bv.g.vol_layout == TT_VOLUME_BRICKS) {
-                    float re, im, wscale, c[3];
-                    splat_source(bv.slices, m, bv.g, s, has_pixel, iy, ix, ccp, re, im, wscale, c);
-                    insert_point_octet(bv.acc, bv.g, re, im, wscale, c, tab[threadIdx.x >> 5], true);
-                } else
-                    insert_point_paired(bv.slices, m, bv.acc, bv.g, s, has_pixel, iy, ix, ccp);
+            for (int first = 0; first < txt; first += 32) {
+                // z-phased filling of large accumulators (the same tiles in every warp)
+                unsigned todo = phase_tiles<TX>(bv.g, m, ty * TY + TY / 2, first, txt, phase, nphase);
+                for (; todo; todo &= todo - 1) {
+                    const int ix = (first + __ffs(todo) - 1) * TX + (lane % TX);
+                    const bool has_pixel = ix < bv.g.wr && iy < bv.g.img_h;
+                    // every lane takes part: lane octets (bricked accumulator) or lane pairs share a pixel
+                    if (bv.g.vol_layout == TT_VOLUME_BRICKS) {
+                        float re, im, wscale, c[3];
+                        splat_source(bv.slices, m, bv.g, s, has_pixel, iy, ix, ccp, re, im, wscale, c);
+                        insert_point_octet(bv.acc, bv.g, re, im, wscale, c, tab[threadIdx.x >> 5], true);
+                    } else {
+                        insert_point_paired(bv.slices, m, bv.acc, bv.g, s, has_pixel, iy, ix, ccp);
+                    }
+                }
             }
         }
         if (threadIdx.x == 0) {

@@ -128,16 +128,16 @@ insert_fixed_kernel(const typename Acc<R>::C* __restrict__ img, const void* __re
     if (threadIdx.x < 9) m[threadIdx.x] = prep_rotation_elem(rot, g.rot_f64, s, threadIdx.x, g, false);
     __syncthreads();
     const FixedSplat sink{acc, fixed_data_scale(*absmax, slices_log2), fixed_weight_scale(slices_log2)};
-    for (int tx = 0; tx < tx_tiles; tx++) {
-        if (nphase > 1 && insert_tile_phase(g, m, min(ty * kTileY + kTileY / 2, g.img_h - 1),
-                                            min(tx * kTileX + kTileX / 2, g.wr - 1), nphase) != phase)
-            continue;
-        int iy, ix;
-        const bool has_pixel = tile_pixel(g, ty * tx_tiles + tx, iy, ix);
-        if constexpr (sizeof(R) == 4)
-            insert_point_fixed_paired(img, m, acc, sink.sd, sink.sw, g, s, has_pixel, iy, ix);  // every lane
-        else if (has_pixel)
-            insert_point_to<R>(img, m, sink, g, s, iy, ix);
+    for (int first = 0; first < tx_tiles; first += 32) {
+        unsigned todo = phase_tiles<kTileX>(g, m, ty * kTileY + kTileY / 2, first, tx_tiles, phase, nphase);
+        for (; todo; todo &= todo - 1) {
+            int iy, ix;
+            const bool has_pixel = tile_pixel(g, ty * tx_tiles + first + __ffs(todo) - 1, iy, ix);
+            if constexpr (sizeof(R) == 4)
+                insert_point_fixed_paired(img, m, acc, sink.sd, sink.sw, g, s, has_pixel, iy, ix);  // every lane
+            else if (has_pixel)
+                insert_point_to<R>(img, m, sink, g, s, iy, ix);
+        }
     }
 }
 

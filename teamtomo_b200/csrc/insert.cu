@@ -54,17 +54,16 @@ insert_accumulate_kernel(const typename Acc<R>::C* __restrict__ img, const void*
     const int ty = blockIdx.x - (int)(s * rows);
     if (threadIdx.x < 9) m[threadIdx.x] = prep_rotation_elem(rot, g.rot_f64, s, threadIdx.x, g, false);
     __syncthreads();
-    for (int tx = 0; tx < tx_tiles; tx++) {
-        // the same answer in every thread: the whole block skips the tile
-        if (nphase > 1 && insert_tile_phase(g, m, min(ty * kTileY + kTileY / 2, g.img_h - 1),
-                                            min(tx * kTileX + kTileX / 2, g.wr - 1), nphase) != phase)
-            continue;
-        int iy, ix;
-        const bool has_pixel = tile_pixel(g, ty * tx_tiles + tx, iy, ix);
-        if constexpr (std::is_same<R, float>::value)
-            insert_point_paired(img, m, acc, g, s, has_pixel, iy, ix);  // every lane takes part
-        else if (has_pixel)
-            insert_point<R>(img, m, acc, g, s, iy, ix);
+    for (int first = 0; first < tx_tiles; first += 32) {
+        unsigned todo = phase_tiles<kTileX>(g, m, ty * kTileY + kTileY / 2, first, tx_tiles, phase, nphase);
+        for (; todo; todo &= todo - 1) {  // the same tiles in every warp
+            int iy, ix;
+            const bool has_pixel = tile_pixel(g, ty * tx_tiles + first + __ffs(todo) - 1, iy, ix);
+            if constexpr (std::is_same<R, float>::value)
+                insert_point_paired(img, m, acc, g, s, has_pixel, iy, ix);  // every lane takes part
+            else if (has_pixel)
+                insert_point<R>(img, m, acc, g, s, iy, ix);
+        }
     }
 }
 
@@ -86,14 +85,14 @@ insert_bricked_kernel(const float2* __restrict__ img, const void* __restrict__ r
     const int iy = ty * kTileY + (threadIdx.x >> 5) * 4 + (lane >> 3);
     const SliceRow row = slice_row_geom(g, m, iy);
     const float2* irow = img + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.slice_pitch;
-    for (int tx = 0; tx < tx_tiles; tx++) {
-        if (nphase > 1 && insert_tile_phase(g, m, min(ty * kTileY + kTileY / 2, g.img_h - 1),
-                                            min(tx * kTileX + kTileX / 2, g.wr - 1), nphase) != phase)
-            continue;
-        const int ix = tx * kTileX + (lane & 7);
-        float re, im, wscale, c[3];
-        splat_source_row(irow, m, row, g, iy < g.img_h && ix < g.wr, ix, re, im, wscale, c);
-        insert_point_octet(acc, g, re, im, wscale, c, tab[threadIdx.x >> 5], false);  // every lane takes part
+    for (int first = 0; first < tx_tiles; first += 32) {
+        unsigned todo = phase_tiles<kTileX>(g, m, ty * kTileY + kTileY / 2, first, tx_tiles, phase, nphase);
+        for (; todo; todo &= todo - 1) {
+            const int ix = (first + __ffs(todo) - 1) * kTileX + (lane & 7);
+            float re, im, wscale, c[3];
+            splat_source_row(irow, m, row, g, iy < g.img_h && ix < g.wr, ix, re, im, wscale, c);
+            insert_point_octet(acc, g, re, im, wscale, c, tab[threadIdx.x >> 5], false);  // every lane takes part
+        }
     }
 }
 
