@@ -93,7 +93,10 @@ batched_slices_kernel(const __grid_constant__ BatchParams bp, unsigned long long
         const int64_t s = local / tyt;  // item = (slice, row of tiles)
         const int ty = (int)(local - s * tyt);
         if (threadIdx.x < 9) m[threadIdx.x] = prep_rotation_elem(bv.rot, bv.g.rot_f64, s, threadIdx.x, bv.g, !INSERT);
-        if (threadIdx.x == 0 && bv.ctf) cc = make_ctf_const(bv.ctf[s]);
+        // the slice's CTF constants: one part each by a lane of warps 1 to 3, beside
+        // warp 0's queue round trip
+        if (bv.ctf && (threadIdx.x & 31) == 0 && threadIdx.x >= 32 && threadIdx.x < 128)
+            make_ctf_const(bv.ctf[s], (threadIdx.x >> 5) - 1, cc);
         // the next item is taken now and published after this one's pixels, so
         // the queue's round trip overlaps the work
         unsigned long long next = 0;

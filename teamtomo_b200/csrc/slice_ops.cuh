@@ -242,27 +242,32 @@ struct CtfConst {
     double inv_px;               // 1 / pixel size (1/Angstrom)
 };
 
-// Constants of one image from its tt_ctf_params (double precision, once per image).
-__host__ __device__ inline CtfConst make_ctf_const(const tt_ctf_params& p) {
-    const double h = 6.62607015e-34, c = 299792458.0, m0 = 9.1093837015e-31, e = 1.602176634e-19;
-    const double volts = (double)p.voltage_kv * 1e3;
-    const double ev = e * volts;
-    const double lambda = h * c / sqrt(ev * (2.0 * m0 * c * c + ev)) * 1e10;  // Angstrom
+// Constants of one image from its tt_ctf_params (double precision, once per
+// image), in three parts of about equal length that different warps form side
+// by side: part 0 the wavelength terms, 1 the phase terms, 2 the astigmatism.
+__device__ inline void make_ctf_const(const tt_ctf_params& p, int part, CtfConst& k) {
     const double pi = 3.14159265358979323846;
-    const double cs = (double)p.spherical_aberration_mm * 1e7;
-    const double ac = (double)p.amplitude_contrast;
-    CtfConst k;
-    k.k1 = -pi * lambda;
-    k.k2 = pi / 2.0 * cs * lambda * lambda * lambda;
-    k.phase = (double)p.phase_shift_deg * pi / 180.0 + atan(ac / sqrt(1.0 - ac * ac));
-    k.defocus = p.defocus_um;
-    k.astig = p.astigmatism_um;
-    const double th = (double)p.astigmatism_angle_deg * pi / 180.0;
-    const double sa = sqrt((double)(p.astigmatism_um > 0 ? p.astigmatism_um : 0.0f));
-    k.ay = sa * sin(th);
-    k.ax = sa * cos(th);
-    k.inv_px = 1.0 / (double)p.pixel_size_a;
-    return k;
+    if (part == 0) {
+        const double h = 6.62607015e-34, c = 299792458.0, m0 = 9.1093837015e-31, e = 1.602176634e-19;
+        const double ev = e * (double)p.voltage_kv * 1e3;
+        const double lambda = h * c / sqrt(ev * (2.0 * m0 * c * c + ev)) * 1e10;  // Angstrom
+        const double cs = (double)p.spherical_aberration_mm * 1e7;
+        k.k1 = -pi * lambda;
+        k.k2 = pi / 2.0 * cs * lambda * lambda * lambda;
+        k.inv_px = 1.0 / (double)p.pixel_size_a;
+    } else if (part == 1) {
+        const double ac = (double)p.amplitude_contrast;
+        k.phase = (double)p.phase_shift_deg * pi / 180.0 + atan(ac / sqrt(1.0 - ac * ac));
+        k.defocus = p.defocus_um;
+    } else {
+        k.astig = p.astigmatism_um;
+        const double th = (double)p.astigmatism_angle_deg * pi / 180.0;
+        const double sa = sqrt((double)(p.astigmatism_um > 0 ? p.astigmatism_um : 0.0f));
+        double sn, cn;
+        sincos(th, &sn, &cn);
+        k.ay = sa * sn;
+        k.ax = sa * cn;
+    }
 }
 
 // CTF at slice frequency (qy, qx) in cycles/pixel.  The phase reaches hundreds
