@@ -59,9 +59,10 @@ __device__ __forceinline__ void load_rotation(float* sm, const void* rot, int64_
 // From the bricked copy the row of tiles is unrolled by four at six resident
 // blocks (40 registers), so one thread's gathers of neighbouring tiles
 // overlap: 256^3 x 4096 1.30 vs 1.32-1.35 ms, 128^3 0.386 vs 0.394 ms.
-// A launch whose rows of tiles do not fill the chip splits each row over
-// gridDim.y blocks (row_splits).
-template <typename VT, int UNR = std::is_same<VT, VoxBrick2>::value ? 4 : 1>
+// SPLIT: a launch whose rows of tiles do not fill the chip splits each row over
+// gridDim.y blocks (row_splits); the bounds known only at run time cost full
+// launches 3 % (256^3 x 4096: 1.26 against 1.23 ms), which go without.
+template <typename VT, bool SPLIT, int UNR = std::is_same<VT, VoxBrick2>::value ? 4 : 1>
 __global__ void __launch_bounds__(kExtractThreads, UNR > 1 ? 6 : 8)
 extract_fwd_kernel(const VT* __restrict__ vol, const void* __restrict__ rot,
                    float2* __restrict__ out, SliceGeom g, int tiles) {
@@ -78,9 +79,9 @@ extract_fwd_kernel(const VT* __restrict__ vol, const void* __restrict__ rot,
     if (iy >= g.img_h) return;
     const SliceRow row = slice_row_geom(g, m, iy);
     float2* orow = out + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.slice_pitch;
-    const int last = split_tile(tx_tiles, blockIdx.y + 1);
+    const int last = SPLIT ? split_tile(tx_tiles, blockIdx.y + 1) : tx_tiles;
 #pragma unroll UNR
-    for (int tx = split_tile(tx_tiles, blockIdx.y); tx < last; tx++) {
+    for (int tx = SPLIT ? split_tile(tx_tiles, blockIdx.y) : 0; tx < last; tx++) {
         const int ix = tx * kTileX + (lane & 7);
         if (ix >= g.wr) continue;
         float qx, c[3];
@@ -476,7 +477,10 @@ static int launch_extract(const VT* vol, const void* rot, float2* out, const Sli
     const int64_t nb = (int64_t)g.n * (tiles / tx_tiles);  // one block per row of tiles, or several
     const bool bricks = std::is_same<VT, VoxBrick2>::value;
     const dim3 grid((unsigned)nb, (unsigned)row_splits(nb, tx_tiles, bricks ? 6 : 8, bricks ? 4 : 1));
-    extract_fwd_kernel<<<grid, kExtractThreads, 0, st>>>(vol, rot, out, g, tiles);
+    if (grid.y > 1)
+        extract_fwd_kernel<VT, true><<<grid, kExtractThreads, 0, st>>>(vol, rot, out, g, tiles);
+    else
+        extract_fwd_kernel<VT, false><<<grid, kExtractThreads, 0, st>>>(vol, rot, out, g, tiles);
     return check_launch("extract_fwd_kernel");
 }
 

@@ -83,6 +83,7 @@ __device__ __forceinline__ void scatter_dv_paired(float2* __restrict__ dvol, con
                                                   float2 gv, bool valid) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, bx = lane & 1;
+    if (!__any_sync(full, valid)) return;  // a patch outside fftfreq_max or the volume
 #pragma unroll
     for (int half = 0; half < 2; half++) {
         const int src = (lane >> 1) + 16 * half;
