@@ -48,6 +48,8 @@ struct BatchParams {
     BatchVolumeDev v[kMaxBatch];
 };
 
+static_assert(sizeof(BatchParams) < 32000, "the descriptors travel as one kernel parameter (32,764 bytes at most)");
+
 template <int TX>
 __host__ inline int tiles_t(int img_h, int wr) {
     constexpr int TY = 256 / TX;

@@ -23,6 +23,8 @@ struct SliceGeom {
     int img_h, wr;  // slice grid rows and rfft columns (h, w/2+1)
     float inv_h, inv_w;            // f32(1/h), f32(1/w)
     float iw0, iw1, s0, s1, sx;    // coordinate scaling of the image/volume shape
+    float riw0, riw1;              // 1 / iw0, 1 / iw1 (divide_by)
+    float half[3], rhalf[3];       // 0.5 n - 0.5 of the volume's axes, and 1 / it
     int D, H, W;                   // rfft volume dims (d, h, w/2+1)
     float ub0, ub1, ub2;           // D-1, H-1, W-1 as float
     int has_fmax;
@@ -54,6 +56,13 @@ __host__ inline SliceGeom make_geom(const tt_slice_params& p) {
     volatile float dd = 1.0f / fd, dh = 1.0f / fh;
     g.iw0 = 1.0f - dd;
     g.iw1 = 1.0f - dh;
+    g.riw0 = 1.0f / g.iw0;
+    g.riw1 = 1.0f / g.iw1;
+    const float dims[3] = {(float)p.vol_d, (float)p.vol_h, (float)p.vol_w};
+    for (int i = 0; i < 3; i++) {
+        g.half[i] = 0.5f * dims[i] - 0.5f;  // both steps exact or rounded alike with and without FMA
+        g.rhalf[i] = 1.0f / g.half[i];
+    }
     g.s0 = fd - 1.0f;
     g.s1 = fh - 1.0f;
     g.sx = fwr - 1.0f;
@@ -110,9 +119,27 @@ __device__ __forceinline__ void rotate_slice_point(const float* m, float qy, flo
     for (int i = 0; i < 3; i++) p[i] = __fadd_rn(__fmul_rn(m[i * 3 + 1], qy), __fmul_rn(m[i * 3 + 2], qx));
 }
 
+// a / b correctly rounded, r the correctly rounded 1 / b: the product a r, then
+// two FMA corrections by the exact remainder a - q b.  The first leaves a
+// faithful quotient (the product alone can be two units off, which is why one
+// correction is not enough), and Markstein's theorem (Brisebarre, Muller and
+// Raina, "Accelerating correctly rounded floating-point division when the
+// divisor is known in advance", IEEE Trans. Computers 53(8), 2004) makes the
+// second correctly rounded.  Compared with IEEE division for every significand
+// of a and the divisors 1 - 1/n and 0.5 n - 0.5 of n = 2 .. 2049: no difference.
+// Five instructions without a branch: 256^3 x 4096 extraction 1.23 -> 1.14 ms.
+// Infinities give NaN, which the callers' range tests refuse alike; a divisor
+// of 0 (an axis of one sample) gives NaN where IEEE division gives one too
+// (0 / 0) or an infinity outside the volume.
+__device__ __forceinline__ float divide_by(float a, float b, float r) {
+    float q = __fmul_rn(a, r);
+    q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
+
 __device__ __forceinline__ void to_dft_coords(const SliceGeom& g, const float p[3], float c[3]) {
-    c[0] = __fmul_rn(__fdiv_rn(__fadd_rn(p[0], 0.5f), g.iw0), g.s0);
-    c[1] = __fmul_rn(__fdiv_rn(__fadd_rn(p[1], 0.5f), g.iw1), g.s1);
+    c[0] = __fmul_rn(divide_by(__fadd_rn(p[0], 0.5f), g.iw0, g.riw0), g.s0);
+    c[1] = __fmul_rn(divide_by(__fadd_rn(p[1], 0.5f), g.iw1, g.riw1), g.s1);
     c[2] = __fmul_rn(__fmul_rn(p[2], 2.0f), g.sx);
 }
 

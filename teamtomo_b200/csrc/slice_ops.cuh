@@ -22,6 +22,14 @@ __device__ __forceinline__ float source_index(float c, float half, float nm1, bo
     return fminf(fmaxf(ix, 0.0f), nm1);
 }
 
+// The same with the reciprocal of half (SliceGeom::half, rhalf).
+__device__ __forceinline__ float source_index(float c, float half, float rhalf, float nm1, bool& grad_ok) {
+    const float gc = __fsub_rn(divide_by(c, half, rhalf), 1.0f);
+    const float ix = __fmul_rn(__fmul_rn(__fadd_rn(gc, 1.0f), 0.5f), nm1);
+    grad_ok = ix > 0.0f && ix < nm1;
+    return fminf(fmaxf(ix, 0.0f), nm1);
+}
+
 struct Corners {
     int z0, y0, x0;
     float ax0, ax1, ay0, ay1, az0, az1;  // per-axis weights of the low/high corner
@@ -38,9 +46,9 @@ struct SourceIdx {
 
 __device__ __forceinline__ SourceIdx source_indices(const SliceGeom& g, const float c[3]) {
     SourceIdx si;
-    si.z = source_index(c[0], 0.5f * (float)g.D - 0.5f, g.ub0, si.gz);
-    si.y = source_index(c[1], 0.5f * (float)g.H - 0.5f, g.ub1, si.gy);
-    si.x = source_index(c[2], 0.5f * (float)g.W - 0.5f, g.ub2, si.gx);
+    si.z = source_index(c[0], g.half[0], g.rhalf[0], g.ub0, si.gz);
+    si.y = source_index(c[1], g.half[1], g.rhalf[1], g.ub1, si.gy);
+    si.x = source_index(c[2], g.half[2], g.rhalf[2], g.ub2, si.gx);
     return si;
 }
 
