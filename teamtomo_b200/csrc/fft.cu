@@ -232,34 +232,39 @@ struct BrickColumnsOut {
     }
 };
 
+// Bricks of the same columns: transform c's fftshifted sample z goes to slot
+// (z & 1, c >> 2, c & 1) of brick (c >> 1) & 1 of the tile's pair, so the eight
+// transforms of a sample fill two whole 32-byte sectors.  Bricks past the row's
+// end are skipped; slots past an odd e get the zeros that absent columns load.
+struct BricksOut {
+    float2* dst;  // slot 0 of the pair's first brick at z = 0
+    int plane, n, bricks;
+    __device__ __forceinline__ void put(int z, int c, float2 v) const {
+        const int t = (c >> 1) & 1;
+        if (t >= bricks) return;
+        float2* o = dst + (int64_t)(z >> 1) * plane + t * 8 + (z & 1) * 4 + (c >> 2) * 2 + (c & 1);
+        *o = v;
+        if (z == n - 1 && !(z & 1)) o[4] = make_float2(0.f, 0.f);
+    }
+};
+
 // z transforms of (d, e, stride) half spectra (y fftshifted) into the bricked copy
 // of the fftshifted (e, e, wr) volume.  A tile is two rows y and four columns
-// x, so its stores are whole pairs of bricks (128-byte lines); slots past an
-// odd e are zero.
+// x.  Storing from the last pass instead of staging the results for 128-byte
+// stores: 320^3 from 160 planes 99 -> 68 us.
 __global__ void __launch_bounds__(kFftMaxThreads, 4)
 columns_to_bricks_kernel(const float2* __restrict__ in, int rows, int off, float2* __restrict__ bricks, int wr,
-                         int stride, int xtiles, const __grid_constant__ FftPlan p) {
+                         int stride, int xtiles, const __grid_constant__ FftPlan p, int smem_tiles) {
     extern __shared__ float2 fft_smem[];
     const int n = p.n, bh = (n + 1) >> 1, bw = (wr + 1) >> 1, tile = fft_tile_size(p);
-    float2 *a = fft_smem, *b = a + tile, *tw = b + tile;
+    float2 *a = fft_smem, *b = a + tile, *tw = a + tile * smem_tiles;
     fft_roots<false>(tw, n);
     const int by = blockIdx.x / xtiles, xt = blockIdx.x - by * xtiles;
     const BrickColumns cols{in + (int64_t)(2 * by) * stride + 4 * xt, (int64_t)n * stride, rows, stride, n - 2 * by,
                             wr - 4 * xt};
-    const PlainTile<true> f{fft_free_tile(a, b, p), n};
-    fft_run<false, true>(Outside<BrickColumns>{cols, off, n}, f, a, b, tw, p);
-    __syncthreads();
-    // slot s of brick t of the pair: z = 2 zb + bit 2, y bit 1, x = 2 t + bit 0
-    const int shift = n - n / 2;  // z (fftshifted) is sample (z + shift) mod n
-    for (int i = threadIdx.x; i < bh * 16; i += blockDim.x) {
-        const int zb = i >> 4, t = (i >> 3) & 1, s = i & 7;
-        if (2 * xt + t >= bw) continue;
-        const int z = 2 * zb + (s >> 2);
-        int k = z + shift;
-        if (k >= n) k -= n;
-        const int q = ((s >> 1) & 1) * 4 + 2 * t + (s & 1);
-        bricks[(((int64_t)zb * bh + by) * bw + 2 * xt + t) * 8 + s] = z < n ? f.at(k, q) : make_float2(0.f, 0.f);
-    }
+    const BricksOut out{bricks + ((int64_t)by * bw + 2 * xt) * 8, bh * bw * 8, n, bw - 2 * xt};
+    // z (fftshifted) is sample (z + n - n / 2) mod n
+    fft_run<false, true>(Outside<BrickColumns>{cols, off, n}, Outside<BricksOut>{out, n - n / 2, n}, a, b, tw, p);
 }
 
 // Insertion accumulators (float4 slots, fftshifted; BRICKED: accumulator_slot
@@ -478,13 +483,14 @@ extern "C" int tt_project_volume_bricks(const float* volumes, int64_t channels, 
                                       st))
         return e;
     size_t sm;
-    if (int e = fft_smem(columns_to_bricks_kernel, b.pe, 2, sm)) return e;
+    const int smem_tiles = fft_tiles(b.pe, false);
+    if (int e = fft_smem(columns_to_bricks_kernel, b.pe, smem_tiles, sm)) return e;
     const int xtiles = (int)((b.wr + 3) / 4), bh = (int)((b.e + 1) / 2);
     const int64_t slots = (int64_t)bh * bh * ((b.wr + 1) / 2) * 8;
     for (int64_t ch = 0; ch < channels; ch++) {
         columns_to_bricks_kernel<<<(unsigned)(bh * xtiles), b.pe.threads, sm, st>>>(
             ys + ch * d * b.e * b.row, (int)d, (int)(at % b.e), (float2*)bricks + ch * slots, (int)b.wr, (int)b.row,
-            xtiles, b.pe);
+            xtiles, b.pe, smem_tiles);
         if (int e = check_launch("columns_to_bricks_kernel")) return e;
     }
     return TT_OK;
