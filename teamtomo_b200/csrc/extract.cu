@@ -62,10 +62,12 @@ __device__ __forceinline__ void load_rotation(float* sm, const void* rot, int64_
 // SPLIT: a launch whose rows of tiles do not fill the chip splits each row over
 // gridDim.y blocks (row_splits); the bounds known only at run time cost full
 // launches 3 % (256^3 x 4096: 1.26 against 1.23 ms), which go without.
-template <typename VT, bool SPLIT, int UNR = std::is_same<VT, VoxBrick2>::value ? 4 : 1>
+// NV volumes `vstride` elements apart are sampled at one pixel's geometry, their
+// slices `ostride` elements apart.
+template <typename VT, bool SPLIT, int NV = 1, int UNR = std::is_same<VT, VoxBrick2>::value ? 4 / NV : 1>
 __global__ void __launch_bounds__(kExtractThreads, UNR > 1 ? 6 : 8)
 extract_fwd_kernel(const VT* __restrict__ vol, const void* __restrict__ rot,
-                   float2* __restrict__ out, SliceGeom g, int tiles) {
+                   float2* __restrict__ out, SliceGeom g, int tiles, int64_t vstride, int64_t ostride) {
     __shared__ float m[9];
     const int tx_tiles = tiles_x_of(g.wr);
     const int rows = tiles / tx_tiles;
@@ -86,13 +88,18 @@ extract_fwd_kernel(const VT* __restrict__ vol, const void* __restrict__ rot,
         if (ix >= g.wr) continue;
         float qx, c[3];
         bool cj = false;
-        float2 r = make_float2(0.0f, 0.0f);
+        float2 r[NV] = {};
         if (extract_geometry_row(g, m, row, ix, qx, cj, c)) {
-            r = sample_trilinear(vol, g, make_corners(g, c));
-            if (cj) r.y = -r.y;
+            const auto k = make_corners(g, c);
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                r[v] = sample_trilinear(vol + v * vstride, g, k);
+                if (cj) r[v].y = -r[v].y;
+            }
         }
         // streaming store: the slices are written once and should not evict the volume from L2
-        __stcs(orow + ix, r);
+#pragma unroll
+        for (int v = 0; v < NV; v++) __stcs(orow + v * ostride + ix, r[v]);
     }
 }
 
@@ -470,26 +477,38 @@ static int launch_backward(const void* v, const void* rot, const float2* gr, flo
     }
 }
 
-template <typename VT>
+template <int NV = 1, typename VT>
 static int launch_extract(const VT* vol, const void* rot, float2* out, const SliceGeom& g, int tiles,
-                          cudaStream_t st) {
+                          cudaStream_t st, int64_t vstride = 0, int64_t ostride = 0) {
     const int tx_tiles = tiles_x_of(g.wr);
     const int64_t nb = (int64_t)g.n * (tiles / tx_tiles);  // one block per row of tiles, or several
     const bool bricks = std::is_same<VT, VoxBrick2>::value;
     const dim3 grid((unsigned)nb, (unsigned)row_splits(nb, tx_tiles, bricks ? 6 : 8, bricks ? 4 : 1));
     if (grid.y > 1)
-        extract_fwd_kernel<VT, true><<<grid, kExtractThreads, 0, st>>>(vol, rot, out, g, tiles);
+        extract_fwd_kernel<VT, true, NV><<<grid, kExtractThreads, 0, st>>>(vol, rot, out, g, tiles, vstride, ostride);
     else
-        extract_fwd_kernel<VT, false><<<grid, kExtractThreads, 0, st>>>(vol, rot, out, g, tiles);
+        extract_fwd_kernel<VT, false, NV><<<grid, kExtractThreads, 0, st>>>(vol, rot, out, g, tiles, vstride, ostride);
     return check_launch("extract_fwd_kernel");
 }
 
-// Slices of a bricked copy, g.slice_rows storage rows of g.slice_pitch elements
-// apart (projections: interleaved channels, padded rows).
-int launch_extract_bricks(const void* bricks, const void* rot, float2* out, const SliceGeom& g, cudaStream_t st) {
+// Slices of `channels` bricked copies of `slots` elements each: (n, channels,
+// img_h, g.slice_pitch) with g.slice_rows rows from slice to slice.  Channels go
+// in pairs, which share the pixel's geometry and corner addresses: two of 320^3
+// at 400 orientations 417 -> 374 us.
+int launch_extract_bricks(const void* bricks, int64_t channels, int64_t slots, const void* rot, float2* out,
+                          const SliceGeom& g, cudaStream_t st) {
     const int tiles = extract_tiles(g);
     if ((int64_t)g.n * tiles > 0x7fffffffLL) return fail(TT_ERR_INVALID, "extract: too many blocks");
-    return launch_extract((const VoxBrick2*)bricks, rot, out, g, tiles, st);
+    const VoxBrick2* vol = (const VoxBrick2*)bricks;
+    const int64_t image = (int64_t)g.img_h * g.slice_pitch;
+    for (int64_t c = 0; c < channels; c += 2) {
+        const VoxBrick2* v = vol + c * slots;
+        float2* o = out + c * image;
+        if (int e = c + 1 < channels ? launch_extract<2>(v, rot, o, g, tiles, st, slots, image)
+                                     : launch_extract(v, rot, o, g, tiles, st))
+            return e;
+    }
+    return TT_OK;
 }
 
 // Bricked copy: voxel (z, y, x), in fftshifted (z, y) order whatever the

@@ -429,7 +429,8 @@ static int make_box(int64_t d, int64_t pad, BoxPlans& b) {
     return TT_OK;
 }
 
-int launch_extract_bricks(const void* bricks, const void* rot, float2* out, const SliceGeom& g, cudaStream_t st);
+int launch_extract_bricks(const void* bricks, int64_t channels, int64_t slots, const void* rot, float2* out,
+                          const SliceGeom& g, cudaStream_t st);
 
 }  // namespace tt
 
@@ -517,10 +518,7 @@ extern "C" int tt_project_slices(const void* bricks, int64_t channels, const voi
     const int64_t count = p->n * channels, half = (b.e + 1) / 2, slots = half * half * ((b.wr + 1) / 2) * 8;
     float2* cs = (float2*)workspace;          // (n, c, d, row)
     float2* slices = cs + count * d * b.row;  // (n, c, e, row)
-    for (int64_t ch = 0; ch < channels; ch++)
-        if (int e = launch_extract_bricks((const float2*)bricks + ch * slots, rotation_matrices,
-                                          slices + ch * b.e * b.row, g, st))
-            return e;
+    if (int e = launch_extract_bricks(bricks, channels, slots, rotation_matrices, slices, g, st)) return e;
     if (int e = launch_columns<true>(slices, Columns{b.e * b.row, b.row, (int)b.e, (int)(b.e - b.e / 2)}, cs,
                                      Columns{d * b.row, b.row, (int)d, (int)(pad + b.e / 2)}, count, (int)b.wr, b.pe,
                                      st))

@@ -110,6 +110,19 @@ def test_reconstruction(d, pad, channels):
     assert a.shape == b.shape and rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 4e-6
 
 
+@pytest.mark.parametrize("d,n,channels", [(33, 5, 2), (32, 5, 3), (16, 6000, 3), (27, 1, 5)])
+def test_channels_match_single_maps(d, n, channels):
+    """Channels are sampled in pairs: a pair, a pair and a rest, launches with whole
+    and with split rows of tiles.  Up to the transforms' rounding (rows of an odd
+    box pair up differently)."""
+    vol = torch.stack([torch.as_tensor(blob_volume(d, seed=i)).float() for i in range(channels)]).cuda()
+    R = torch.as_tensor(rotations(n, seed=4)).float().cuda()
+    got = tt().project_3d_to_2d_multichannel(vol, R)
+    for c in range(channels):
+        ref = tt().project_3d_to_2d(vol[c], R)
+        assert rel_l2(got[:, c].cpu().numpy(), ref.cpu().numpy()) < 4e-6
+
+
 def test_unsupported_boxes_keep_the_general_path(monkeypatch):
     """A prime factor above 13 (68 = 4 * 17) and float64 maps."""
     assert not _own(34, 2.0) and not _own(600, 2.0)
