@@ -92,8 +92,27 @@ inline size_t fft_smem_bytes(const FftPlan& p, int tiles) {
     return ((size_t)p.pitched * kFftBatch * tiles + p.n) * sizeof(float2);
 }
 
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Both components in one instruction: the transforms are bound by issue slots
+// (65 %).  With the column passes' twiddles from memory: columns of 800 x 320^2
+// 138 -> 131 us, 320^3 from 160 planes 67 -> 65 us.
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+    float2 r;
+    asm("{ .reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; add.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+    float2 r;
+    asm("{ .reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; sub.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+// a + t and a - t for a t whose components were swapped (turn): one by one, as a
+// pair they would have to be moved first.
+__device__ __forceinline__ float2 cadd1(float2 a, float2 t) { return make_float2(a.x + t.x, a.y + t.y); }
+__device__ __forceinline__ float2 csub1(float2 a, float2 t) { return make_float2(a.x - t.x, a.y - t.y); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
@@ -197,8 +216,8 @@ struct Dft {
                 b.y = fmaf(s, u[m - 1].y, b.y);
             }
             const float2 w = turn<INV>(b);
-            y[q] = cadd(a, w);
-            y[R - q] = csub(a, w);
+            y[q] = cadd1(a, w);
+            y[R - q] = csub1(a, w);
         }
 #pragma unroll
         for (int q = 0; q < R; q++) v[q] = y[q];
@@ -218,9 +237,9 @@ struct Dft<4, INV> {
         const float2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]), c = cadd(v[1], v[3]);
         const float2 d = turn<INV>(csub(v[1], v[3]));
         v[0] = cadd(a, c);
-        v[1] = cadd(b, d);
+        v[1] = cadd1(b, d);
         v[2] = csub(a, c);
-        v[3] = csub(b, d);
+        v[3] = csub1(b, d);
     }
 };
 
@@ -332,7 +351,7 @@ struct Dft<20, INV> : DftCoprime<4, 5, INV> {};
 //
 // A pass reads butterfly j's samples j + r * nb (nb = n / R) from a source and
 // writes results o + r * ns to a destination.  Sources and destinations give a
-// cursor for one butterfly, then take r.
+// cursor for one butterfly, then take r (and, to read, the radix).
 
 // A tile in natural order.
 template <bool COLUMNS>
@@ -343,7 +362,7 @@ struct PlainTile {
     struct Cursor {
         float2* t;
         int step;
-        __device__ __forceinline__ float2 get(int r) const { return t[r * step]; }
+        __device__ __forceinline__ float2 get(int r, int) const { return t[r * step]; }
         __device__ __forceinline__ void put(int r, float2 v) const { t[r * step] = v; }
     };
     __device__ __forceinline__ Cursor from(int j, int c, int nb, const FftPlan&) const {
@@ -391,7 +410,7 @@ struct Outside {
             const int y = x + r * step;  // in [0, 2 n)
             return (int)min((unsigned)y, (unsigned)(y - n));
         }
-        __device__ __forceinline__ float2 get(int r) const { return f.get(where(r), c); }
+        __device__ __forceinline__ float2 get(int r, int) const { return f.get(where(r), c); }
         __device__ __forceinline__ void put(int r, float2 v) const { f.put(where(r), c, v); }
     };
     __device__ __forceinline__ int back(int k) const {
@@ -408,8 +427,9 @@ struct Outside {
 
 // One Stockham pass of radix R.  Consecutive threads take the eight transforms
 // of one butterfly (COLUMNS) or consecutive butterflies of one transform.
-// Twiddles: the roots of powers r = 1, 2, 4, .. are read, the others are
-// products of at most four of them.
+// Twiddles are read by the column passes (four addresses a warp).  In the row
+// passes, where they would conflict, the roots of powers r = 1, 2, 4, .. are read
+// and the others are products of at most four of them.
 template <int R, bool INV, bool COLUMNS, bool FIRST, class Src, class Dst>
 __device__ __forceinline__ void fft_pass(const Src& src, const Dst& dst, const float2* tw, const FftPlan& p, int s) {
     const int nb = p.n / R, ns = FIRST ? 1 : p.ns[s];
@@ -420,13 +440,13 @@ __device__ __forceinline__ void fft_pass(const Src& src, const Dst& dst, const f
         float2 v[R];
         const auto in = src.from(j, c, nb, p);
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = in.get(r);
+        for (int r = 0; r < R; r++) v[r] = in.get(r, R);
         if constexpr (!FIRST) {
             float2 w[R];
             const int at = k * p.step[s];
 #pragma unroll
             for (int r = 1; r < R; r++) {
-                const int top = r >= 16 ? 16 : (r >= 8 ? 8 : (r >= 4 ? 4 : (r >= 2 ? 2 : 1)));
+                const int top = COLUMNS ? r : r >= 16 ? 16 : (r >= 8 ? 8 : (r >= 4 ? 4 : (r >= 2 ? 2 : 1)));
                 w[r] = r == top ? tw[r * at] : cmul(w[top], w[r - top]);
                 v[r] = cmul(v[r], w[r]);
             }
