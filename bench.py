@@ -775,7 +775,7 @@ def config_workload(args):
         out.update({"metric": "slices/s project_3d_to_2d 64^3 pad 2.0", "value": k / (ms / 1e3), "unit": "slices/s",
                     "ms_per_step": ms, "config": {"workload": "project 64^3 x 100 rotations, pad 2.0"},
                     "torch_gpu_reference": None if ref is None else {"value": k / (ref_ms / 1e3), "ms": ref_ms},
-                    "cpu_baseline": cpu, "clocks": clk, "gpu_launches": 4 * args.steps})
+                    "cpu_baseline": cpu, "clocks": clk, "gpu_launches": 7 * args.steps})
     elif args.workload == "backproject":
         n, k = 128, 10_000
         vol = blob_volume_torch(n, 1002, dev)
@@ -818,7 +818,7 @@ def config_workload(args):
                     "config": {"workload": "backproject 10,000 x 128^2 (SNR 0.1); value at pad 1.0 "
                                "(128x128x65 volume), pad 2.0 beside it"},
                     "pads": res, "torch_gpu_reference": refres, "cpu_baseline": cpu, "clocks": clk,
-                    "gpu_launches": 5 * args.steps})
+                    "gpu_launches": 7 * args.steps})
     else:
         n, n_img, n_ext, chunk = 320, 200_000, 100_000, 10_000
         vol_real = blob_volume_torch(n, 1005, dev)
@@ -944,7 +944,7 @@ def kernel_case(name, dev):
         T = crandn(ns, n, n // 2 + 1)
         det = name == "det_insert"
         return (lambda: tt.insert_central_slices_rfft_3d(T, shape, R, deterministic=det)), \
-            ns * 8 * P + 12 * vox, "insert_accumulate_kernel / insert_fixed_kernel + finalize"
+            ns * 8 * P + 12 * vox, "insert_bricked_kernel / insert_fixed_kernel + finalize"
     if name == "insert_bwd":
         T = crandn(ns, n, n // 2 + 1).requires_grad_(True)
         H = crandn(n, n, n // 2 + 1)
@@ -1032,14 +1032,15 @@ def kernel_case_more(name, dev, V, R, crandn, gen):
         # non-FFT bytes: pad x sinc^2 (read b^3, write (2b)^3), extraction (write k (2b)(b+1)),
         # recentre / crop (read k (2b)^2, write k b^2), all float32 / complex64
         return (lambda: tt.project_3d_to_2d(vol, Rp)), 4 * b ** 3 + 4 * (2 * b) ** 3 + k * 8 * 2 * b * (b + 1) + \
-            k * 4 * ((2 * b) ** 2 + b * b), "project_prepare_kernel, extraction, recentre_crop_2d_kernel"
+            k * 4 * ((2 * b) ** 2 + b * b), \
+            "sinc2_kernel, rows_r2c_kernel, columns_kernel, columns_to_bricks_kernel, extraction, rows_c2r_kernel"
     if name == "backproject":
         b, k = 128, 2048
         imgs = torch.randn((k, b, b), device=dev, generator=gen)
         Rp = torch.tensor(rotations(k, 1002), device=dev)
         return (lambda: tt.backproject_2d_to_3d(imgs, Rp)), k * 4 * (b * b + (2 * b) ** 2) + k * 8 * 2 * b * (
             b + 1) + 20 * (2 * b) ** 2 * (b + 1) + 8 * (2 * b) ** 3, \
-            "pad_fftshift_2d_kernel, insertion, normalize_unshift_kernel, backproject_finish_kernel"
+            "rows_r2c_kernel, columns_kernel, insertion, normalize_columns_kernel, rows_c2r_kernel, sinc2_kernel"
     if name == "pack_bricks":
         p = slice_params(n=1, image_shape=(n, n, n), volume=V, rotation=R)
         return (lambda: _layout.pack(V, p, _layout.BRICKS)), 16 * vox, "pack_bricks_kernel"

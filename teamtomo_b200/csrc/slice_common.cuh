@@ -8,7 +8,8 @@
 //   * array coordinates: ((p + 0.5) / (1 - 1/n)) * (n - 1) for z and y,
 //                        (p * 2) * (w/2 + 1 - 1) for x
 //                        (torch_fourier_slice/_dft_utils.py:37-72)
-// __fmul_rn / __fadd_rn / __fdiv_rn keep nvcc from contracting into FMAs.
+// __fmul_rn / __fadd_rn keep nvcc from contracting into FMAs; the divisions, by
+// constants of the box, are correctly rounded (divide_by).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -2,7 +2,11 @@
 
 Same steps as torch_fourier_slice/backproject.py:11-92 — pad, 2D rfft,
 central-slice insertion, division by max(weights, 1), 3D irfft, division by
-sinc^2, crop — with the fftshifts folded into kernel addressing: one kernel
+sinc^2, crop — with the fftshifts folded into kernel addressing.  Untracked
+float32 images of supported boxes run on the library's own transforms
+(_reconstruct), which skip the zeros of the padding and the rows that the crop
+drops, and apply the completion and the normalisation while they load the
+accumulator.  The others: one kernel
 pads and shifts the images, the insertion reads the unshifted 2D rfft, one
 kernel applies the Friedel completion, the normalisation and the inverse
 shift, and one kernel recentres, divides by sinc^2 and crops.

@@ -2,10 +2,17 @@
 
 Same steps as torch_fourier_slice/project.py:12-93 — pad, premultiply by
 sinc^2, 3D rfft, central-slice extraction, 2D irfft, crop — with the fftshift
-bookkeeping folded into the kernels' addressing: the padded, sinc^2-weighted
-volume is written directly in FFT order by one kernel, the extraction reads
-the unshifted rfftn output and writes rows already ifftshifted for the 2D
-irfft, and one kernel recentres and crops the projections.
+bookkeeping folded into the kernels' addressing.
+
+Single precision boxes whose padded size has factors the library's transforms
+support (_own_transforms) never exist padded: the transforms read the zeros
+as absent rows, write the spectrum as the bricked copy that the extraction
+gathers from, and invert only the rows and columns that the crop keeps.
+
+The others take the general path: the padded, sinc^2-weighted volume is
+written in FFT order by one kernel, the extraction reads the unshifted rfftn
+output and writes rows already ifftshifted for the 2D irfft, and one kernel
+recentres and crops the projections.
 """
 
 from __future__ import annotations
@@ -43,10 +50,10 @@ def _out_dtype(volume: torch.Tensor) -> torch.dtype:
 
 
 # CUDA-graph replay of small projections.  A projection of a small volume is
-# a chain of about ten short kernels (the padding / sinc^2 pass, the 3D rfft,
-# the extraction, the 2D inverse FFTs, the crop) whose host-side launch cost
-# exceeds their GPU time: 64^3 at pad 2, 100 rotations took 220 us per call
-# eagerly and 122 us as one graph replay on a B200.  Calls without autograd on
+# a chain of short kernels (sinc^2, the 3D transform, the extraction, the 2D
+# inverse transforms) whose host-side launch cost exceeds their GPU time: 64^3
+# at pad 2, 100 rotations take 78 us per call eagerly and 60 us as one graph
+# replay on a B200 (220 and 122 us on the general path's longer chain).  Calls without autograd on
 # small volumes therefore replay a graph captured once per (device, shapes,
 # dtypes, arguments), copying the inputs into its static buffers and cloning
 # the output; ``TT_PROJECT_GRAPHS=0`` turns this off.
