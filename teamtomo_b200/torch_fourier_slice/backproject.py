@@ -89,7 +89,9 @@ def _backproject(images, rotation_matrices, pad_factor, fftfreq_max, zyx_matrice
     c = images.shape[-3] if channels else 1
     flat = _lib.dense(images.reshape(-1, d, d))
     track = torch.is_grad_enabled() and images.requires_grad
-    if (not track and images.dtype == torch.float32 and nrot * c == flat.shape[0] > 0
+    # images that any derivative can be asked of (forward mode and functorch
+    # too) go through the autograd Functions; the rotations are constants here
+    if (_lib.untracked(images) and images.dtype == torch.float32 and nrot * c == flat.shape[0] > 0
             and _lib.load().tt_transform_supported(d, p)):
         out = _reconstruct(flat, R, c, p, fftfreq_max, zyx_matrices)
         return out if channels else out[0]
