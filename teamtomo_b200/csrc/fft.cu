@@ -409,7 +409,8 @@ template <typename K>
 static int fft_smem(K kernel, const FftPlan& p, int tiles, size_t& bytes) {
     bytes = fft_smem_bytes(p, tiles);
     if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        // always the same limit: a thread must not lower it between another one's call and launch
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFftSmemLimit);
         if (e != cudaSuccess) return fail(TT_ERR_CUDA, "transform: shared memory: %s", cudaGetErrorString(e));
     }
     return TT_OK;

@@ -91,6 +91,7 @@ __device__ __forceinline__ int fft_tile_size(const FftPlan& p) { return p.pitche
 inline size_t fft_smem_bytes(const FftPlan& p, int tiles) {
     return ((size_t)p.pitched * kFftBatch * tiles + p.n) * sizeof(float2);
 }
+constexpr int kFftSmemLimit = 227 * 1024;  // a block's most; two tiles of 1000 samples take 145 KB
 
 // Both components in one instruction: the transforms are bound by issue slots
 // (65 %).  With the column passes' twiddles from memory: columns of 800 x 320^2
