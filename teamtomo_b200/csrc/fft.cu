@@ -47,11 +47,11 @@ namespace tt {
 // (n, n, n2) array, times (DIV: over) the array's sinc(|f|)^2.  One warp per
 // row: its two leading frequencies are formed once.  A pass of its own because
 // the weight costs more than a transform's step per sample and the transform
-// kernels hold their samples in registers.
+// kernels hold their samples in registers.  `out` may be `in`.
 template <bool DIV>
 __global__ void __launch_bounds__(256)
-sinc2_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t rows, int d, int len, int pad, int n,
-             int n2, float inv_n, float inv_n2) {
+sinc2_kernel(const float* in, float* out, int64_t rows, int d, int len, int pad, int n, int n2, float inv_n,
+             float inv_n2) {
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int r = (int)(row % ((int64_t)d * d));
