@@ -281,7 +281,8 @@ int32_t tt_insert_prefers_bricks(const tt_slice_params *p);
 
 /* Adds channel-interleaved slices (n, channels, h, pitch) complex64, w/2+1 of
  * each row's `pitch` elements used, to `channels` float accumulators back to
- * back, plain or `bricked`; every channel gets the weights. */
+ * back, plain or `bricked` (fewer than 2^31 slots each); every channel gets the
+ * weights. */
 int tt_insert_accumulate_rows(const void *image_rfft, int64_t channels, int64_t pitch,
                               const void *rotation_matrices, void *accumulator, int32_t bricked,
                               const tt_slice_params *p, void *stream);

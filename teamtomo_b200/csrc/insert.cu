@@ -468,6 +468,8 @@ extern "C" int tt_insert_accumulate_rows(const void* image_rfft, int64_t channel
         return fail(TT_ERR_INVALID, "insert_accumulate_rows: a row holds at least w/2 + 1 elements");
     if (p->deterministic || p->volume_unshifted)
         return fail(TT_ERR_INVALID, "insert_accumulate_rows: a float accumulator of an fftshifted volume");
+    if (bricked && !bricks_fit(p))
+        return fail(TT_ERR_INVALID, "insert_accumulate_rows: a bricked accumulator must hold fewer than 2^31 slots");
     if (p->n == 0) return TT_OK;
     if (!image_rfft || !rotation_matrices || !accumulator)
         return fail(TT_ERR_INVALID, "insert_accumulate_rows: NULL pointer argument");
