@@ -74,48 +74,76 @@ __device__ __forceinline__ float2* fft_free_tile(float2* a, float2* b, const Fft
 // channels, orientations), so an image comes out as it would alone.  ODD: the
 // images have an odd number of rows, each one's last row goes with zeros, and a
 // tile's pairs may belong to several images.  With an even number (and for one
-// image) consecutive rows never straddle.  4000 projections of 33^3 at pad 2
-// 211 us either way, 4000 reconstructed images of 33^2 361 -> 368 us (3 % more
-// transforms), of 113^2 at 600 images 595 -> 593 us.
+// image) consecutive rows never straddle.  Row transforms, pairs of the launch /
+// pairs of an image: 4000 images of 33^2 33.0 / 34.8 us (3 % more transforms),
+// of 45^2 29.5 / 31.5, 600 of 113^2 40.3 / 36.2; inverse ones of 8000 images of
+// 33^2 34.6 / 34.9, of 45^2 47.0 / 49.3, 1200 of 113^2 60.5 / 60.9.
 struct RowPairs {
     int64_t count;  // rows; pairs when ODD
     uint32_t per;   // ODD: pairs of an image
-    uint32_t inv;   // ODD: floor(2^16 / per) + 1 below eight pairs (i / per = i * inv >> 16 for i < 8), else 0
+    uint32_t inv;   // ODD: floor((2^32 - 1) / per)
 };
 inline RowPairs make_row_pairs(int64_t images, int64_t rows, bool& odd) {
     odd = images > 1 && (rows & 1);
     if (!odd) return RowPairs{images * rows, 1, 0};
-    const int64_t per = (rows + 1) / 2;
-    return RowPairs{images * per, (uint32_t)per, per < kFftBatch ? 65536 / (uint32_t)per + 1 : 0};
+    const uint32_t per = (uint32_t)((rows + 1) / 2);
+    return RowPairs{images * per, per, 0xffffffffu / per};
 }
 
-// The rows of tile t's transforms: c takes rows row(c) and row(c) + 1 from the
-// tile's first row on, the ones that exist.
+// A transform's rows, `at` and a row length further: the offset from the tile's
+// first row (RowTile::first) and which exist.
+struct RowPair {
+    int at;
+    bool one, two;
+};
+
+// The rows of a tile's transforms.  of(c, len) is what a butterfly keeps of
+// transform c: its index, or (ODD) its pair, which formed again for each sample
+// costs 5 % there; kept, it costs even tiles 2 to 4 %.
 template <bool ODD>
 struct RowTile {
-    int left;        // rows left, pairs left when ODD
-    uint32_t k, per, inv;  // ODD: index of the tile's first pair in its image
-    __device__ __forceinline__ RowTile(const RowPairs& p, int64_t t, int64_t& first) : k(0), per(p.per), inv(p.inv) {
-        if (ODD) {
-            const uint32_t pair = (uint32_t)t * kFftBatch, image = pair / per;  // fewer than 2^32 pairs
-            k = pair - image * per;
-            first = 2 * (int64_t)pair - image;
-            left = (int)min((int64_t)kFftBatch, p.count - pair);
-        } else {
-            first = t * (2 * kFftBatch);
-            left = (int)min((int64_t)(2 * kFftBatch), p.count - first);
+    int left;  // rows left
+    static __device__ __forceinline__ int64_t first(const RowPairs&, int64_t t) { return t * (2 * kFftBatch); }
+    __device__ __forceinline__ RowTile(const RowPairs& p, int64_t t)
+        : left((int)min((int64_t)(2 * kFftBatch), p.count - t * (2 * kFftBatch))) {}
+    __device__ __forceinline__ int of(int c, int) const { return c; }
+    __device__ __forceinline__ RowPair pair(int c, int len) const {
+        return RowPair{2 * c * len, 2 * c < left, 2 * c + 1 < left};
+    }
+};
+template <>
+struct RowTile<true> {
+    int left;        // pairs left
+    uint32_t table;  // four bits a transform: images that end before it, whether one ends with it
+    // Image of the tile's first pair (of fewer than 2^32) and the pair's place in it.
+    static __device__ __forceinline__ uint32_t image(const RowPairs& p, int64_t t, uint32_t& k) {
+        const uint32_t pair = (uint32_t)t * kFftBatch;
+        uint32_t i = __umulhi(pair, p.inv);  // at most one too low
+        k = pair - i * p.per;
+        if (k >= p.per) {
+            i++;
+            k -= p.per;
         }
+        return i;
     }
-    // images that end before transform c
-    __device__ __forceinline__ uint32_t ends(int c) const {
-        const uint32_t i = k + c;
-        return i < per ? 0 : 1 + (((i - per) * inv) >> 16);
+    static __device__ __forceinline__ int64_t first(const RowPairs& p, int64_t t) {
+        uint32_t k;
+        return 2 * kFftBatch * t - image(p, t, k);
     }
-    __device__ __forceinline__ int row(int c) const { return ODD ? 2 * c - (int)ends(c) : 2 * c; }
-    __device__ __forceinline__ bool one(int c) const { return ODD ? c < left : 2 * c < left; }
-    __device__ __forceinline__ bool two(int c) const {
-        return ODD ? c < left && k + c + 1 != (ends(c) + 1) * per : 2 * c + 1 < left;
+    __device__ __forceinline__ RowTile(const RowPairs& p, int64_t t)
+        : left((int)min((int64_t)kFftBatch, p.count - t * kFftBatch)), table(0) {
+        uint32_t k;
+        image(p, t, k);
+        // the pairs that end an image: one at most from eight pairs an image up
+        for (uint32_t end = p.per - k; end <= kFftBatch; end += p.per)
+            table += ((0x11111111u << (4 * (end - 1))) << 4) + (8u << (4 * (end - 1)));
     }
+    __device__ __forceinline__ RowPair of(int c, int len) const {
+        const int t = (int)(table >> (4 * c));
+        return RowPair{(2 * c - (t & 7)) * len, c < left, c < left && !(t & 8)};
+    }
+    __device__ __forceinline__ RowPair pair(const RowPair& r, int) const { return r; }
+    __device__ __forceinline__ RowPair pair(int c, int len) const { return of(c, len); }
 };
 
 template <bool ODD>
@@ -123,12 +151,15 @@ struct RealRows {
     const float* src;
     int len;
     RowTile<ODD> rows;
-    __device__ __forceinline__ float2 get(int x, int c) const {
+    __device__ __forceinline__ auto of(int c) const { return rows.of(c, len); }
+    template <class C>
+    __device__ __forceinline__ float2 get(int x, const C& c) const {
         float2 v = make_float2(0.f, 0.f);
         if (x < len) {
-            const int at = rows.row(c) * len + x;
-            if (rows.one(c)) v.x = __ldcs(src + at);
-            if (rows.two(c)) v.y = __ldcs(src + at + len);
+            const RowPair r = rows.pair(c, len);
+            const int at = r.at + x;
+            if (r.one) v.x = __ldcs(src + at);
+            if (r.two) v.y = __ldcs(src + at + len);
         }
         return v;
     }
@@ -139,11 +170,14 @@ struct RealRowsOut {
     int len;
     RowTile<ODD> rows;
     float scale;
-    __device__ __forceinline__ void put(int x, int c, float2 v) const {
+    __device__ __forceinline__ auto of(int c) const { return rows.of(c, len); }
+    template <class C>
+    __device__ __forceinline__ void put(int x, const C& c, float2 v) const {
         if (x >= len) return;
-        const int at = rows.row(c) * len + x;
-        if (rows.one(c)) dst[at] = v.x * scale;
-        if (rows.two(c)) dst[at + len] = v.y * scale;
+        const RowPair r = rows.pair(c, len);
+        const int at = r.at + x;
+        if (r.one) dst[at] = v.x * scale;
+        if (r.two) dst[at + len] = v.y * scale;
     }
 };
 
@@ -178,8 +212,9 @@ struct HalfSpectra {
         }
     };
     __device__ __forceinline__ Cursor from(int j, int c, int nb, const FftPlan&) const {
-        const float2* row = src + rows.row(c) * stride;
-        return Cursor{row + j, row + n - j, j, nb, n, stride, edge, rows.one(c), rows.two(c)};
+        const RowPair r = rows.pair(c, stride);
+        const float2* row = src + r.at;
+        return Cursor{row + j, row + n - j, j, nb, n, stride, edge, r.one, r.two};
     }
 };
 
@@ -188,6 +223,7 @@ struct ColumnRows {
     const float2* src;
     int64_t row;
     int rows, cols;
+    __device__ __forceinline__ int of(int c) const { return c; }
     __device__ __forceinline__ float2 get(int r, int c) const {
         return (r < rows && c < cols) ? __ldcs(src + r * row + c) : make_float2(0.f, 0.f);
     }
@@ -196,6 +232,7 @@ struct ColumnRowsOut {
     float2* dst;
     int64_t row;
     int rows, cols;
+    __device__ __forceinline__ int of(int c) const { return c; }
     __device__ __forceinline__ void put(int r, int c, float2 v) const {
         if (r < rows && c < cols) dst[r * row + c] = v;
     }
@@ -215,8 +252,8 @@ rows_r2c_kernel(const float* __restrict__ in, float2* __restrict__ out, RowPairs
     fft_roots<false>(tw, n);
     const PlainTile<false> z{fft_free_tile(a, b, p), n};
     for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        int64_t first;
-        const RowTile<ODD> rows(pairs, t, first);
+        const RowTile<ODD> rows(pairs, t);
+        const int64_t first = RowTile<ODD>::first(pairs, t);
         const RealRows<ODD> rows_in{in + first * len, len, rows};
         fft_run<false, false>(Outside<RealRows<ODD>>{rows_in, off, n}, z, a, b, tw, p);
         __syncthreads();
@@ -225,13 +262,14 @@ rows_r2c_kernel(const float* __restrict__ in, float2* __restrict__ out, RowPairs
         // images of 128^2 657 -> 631 us)
         for (int w = threadIdx.x >> 5; w < (wr + 31) / 32 * kFftBatch; w += blockDim.x >> 5) {
             const int c = w & (kFftBatch - 1), k = w / kFftBatch * 32 + (threadIdx.x & 31);
-            if (k >= wr || !rows.one(c)) continue;
+            const RowPair r = rows.pair(c, stride);
+            if (k >= wr || !r.one) continue;
             const float2 u = z.at(k, c), m = z.at(k ? n - k : 0, c);
             const float f = 0.5f * (k == 0 || 2 * k == n ? edge : inner);
             // Z = X1 + i X2: X1 = (Z[k] + conj Z[n-k]) / 2, X2 = (Z[k] - conj Z[n-k]) / 2i
-            const int at = rows.row(c) * stride + k;
+            const int at = r.at + k;
             dst[at] = make_float2(f * (u.x + m.x), f * (u.y - m.y));
-            if (rows.two(c)) dst[at + stride] = make_float2(f * (u.y + m.y), f * (m.x - u.x));
+            if (r.two) dst[at + stride] = make_float2(f * (u.y + m.y), f * (m.x - u.x));
         }
         __syncthreads();
     }
@@ -250,8 +288,8 @@ rows_c2r_kernel(const float2* __restrict__ in, float* __restrict__ out, RowPairs
     float2 *a = fft_smem, *b = a + tile, *tw = a + tile * smem_tiles;
     fft_roots<true>(tw, n);
     for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        int64_t first;
-        const RowTile<ODD> rows(pairs, t, first);
+        const RowTile<ODD> rows(pairs, t);
+        const int64_t first = RowTile<ODD>::first(pairs, t);
         const HalfSpectra<ODD> spectra{in + first * stride, stride, n, 1.0f / inner, rows};
         const RealRowsOut<ODD> rows_out{out + first * len, len, rows, scale * inner};
         fft_run<true, false>(spectra, Outside<RealRowsOut<ODD>>{rows_out, off, n}, a, b, tw, p);
@@ -292,6 +330,7 @@ struct BrickColumns {
     const float2* src;
     int64_t row;
     int rows, stride, ys, xs;
+    __device__ __forceinline__ int of(int c) const { return c; }
     __device__ __forceinline__ float2 get(int r, int c) const {
         return (r < rows && (c >> 2) < ys && (c & 3) < xs) ? __ldcs(src + r * row + (c >> 2) * stride + (c & 3))
                                                           : make_float2(0.f, 0.f);
@@ -301,6 +340,7 @@ struct BrickColumnsOut {
     float2* dst;
     int64_t row;
     int rows, stride, ys, xs;
+    __device__ __forceinline__ int of(int c) const { return c; }
     __device__ __forceinline__ void put(int r, int c, float2 v) const {
         if (r < rows && (c >> 2) < ys && (c & 3) < xs) dst[r * row + (c >> 2) * stride + (c & 3)] = v;
     }
@@ -313,6 +353,7 @@ struct BrickColumnsOut {
 struct BricksOut {
     float2* dst;  // slot 0 of the pair's first brick at z = 0
     int plane, n, bricks;
+    __device__ __forceinline__ int of(int c) const { return c; }
     __device__ __forceinline__ void put(int z, int c, float2 v) const {
         const int t = (c >> 1) & 1;
         if (t >= bricks) return;

@@ -398,15 +398,17 @@ struct PitchedTile {
     }
 };
 
-// Global memory: f.get(x, c) / f.put(x, c, v) with x = (sample - off) mod n, the
-// row or column behind a sample.
+// Global memory: f.get(x, f.of(c)) / f.put(x, f.of(c), v) with x = (sample -
+// off) mod n, the row or column behind a sample; of(c) is what f keeps of a
+// transform for a whole butterfly (its index, or more).
 template <class F>
 struct Outside {
     const F& f;
     int off, n;
     struct Cursor {
         const F& f;
-        int x, step, n, c;
+        int x, step, n;
+        decltype(f.of(0)) c;
         __device__ __forceinline__ int where(int r) const {
             const int y = x + r * step;  // in [0, 2 n)
             return (int)min((unsigned)y, (unsigned)(y - n));
@@ -419,10 +421,10 @@ struct Outside {
         return x < 0 ? x + n : x;
     }
     __device__ __forceinline__ Cursor from(int j, int c, int nb, const FftPlan&) const {
-        return Cursor{f, back(j), nb, n, c};
+        return Cursor{f, back(j), nb, n, f.of(c)};
     }
     __device__ __forceinline__ Cursor to(int j, int k, int c, int R, const FftPlan& p, int s) const {
-        return Cursor{f, back((j - k) * R + k), p.ns[s], n, c};
+        return Cursor{f, back((j - k) * R + k), p.ns[s], n, f.of(c)};
     }
 };
 
