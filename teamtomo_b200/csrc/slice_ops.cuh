@@ -678,8 +678,10 @@ __device__ __forceinline__ void insert_point_octet(float4* __restrict__ acc, con
         const float w = (fmaf(f.x, az, bz) * fmaf(f.y, ay, by)) * fmaf(f.z, ax, bx);
         const uint32_t slot = base + ((base & 4u) ? oz : ez) + ((base & 2u) ? oy : ey) + ((base & 1u) ? ox : ex);
         // a corner of zero weight adds nothing, whatever the data and the CTF: past
-        // the last index its slot is not its voxel's (0 * NaN would reduce into it)
-        float re = w != 0.0f ? d.x * w : 0.0f, im = w != 0.0f ? d.y * w : 0.0f, wt = w != 0.0f ? w * f.w : 0.0f;
+        // the last index its slot is not its voxel's (0 * NaN would reduce into it;
+        // without a CTF the scale is 0 or 1)
+        float re = w != 0.0f ? d.x * w : 0.0f, im = w != 0.0f ? d.y * w : 0.0f;
+        float wt = !ctf || w != 0.0f ? w * f.w : 0.0f;
         const bool shared = (code >> corner) & 1;
         const int from = other + ((code >> 8) & 15);
         const float ore = __shfl_sync(full, re, from), oim = __shfl_sync(full, im, from),
