@@ -982,16 +982,16 @@ def kernel_case_more(name, dev, V, R, crandn, gen):
                 "batched_slices_kernel<extract>"
         sl = B.extract_central_slices_rfft_3d_batched(vols, rots, ctf=ctfs)
         return (lambda: B.insert_central_slices_rfft_3d_batched(sl, rots, ctf=ctfs)), slice_bytes + 12 * vb, \
-            "batched_slices_kernel<insert> + insert_finalize_kernel"
+            "batched_slices_kernel<insert> + finalize of each volume"
     if name in ("sample3d", "insert3d"):
         m = 1 << 24
         img = torch.randn((n, n, n), device=dev, generator=gen)
         coords = torch.rand((m, 3), device=dev, generator=gen) * (n - 1)
         if name == "sample3d":
-            return (lambda: tt.sample_image_3d(img, coords)), 4 * n ** 3 + 16 * m, "sample3d_kernel"
+            return (lambda: tt.sample_image_3d(img, coords)), 4 * n ** 3 + 16 * m, "sample3d_f32_kernel"
         vals = torch.randn(m, device=dev, generator=gen)
         return (lambda: tt.insert_into_image_3d(vals, coords, torch.zeros_like(img))), 16 * m + 8 * n ** 3, \
-            "insert3d_kernel"
+            "splat_bricked_kernel + splat_finish_kernel"
     if name == "affine3d":
         img = torch.randn((n, n, n), device=dev, generator=gen)
         M = torch.eye(4, device=dev)
@@ -1029,17 +1029,15 @@ def kernel_case_more(name, dev, V, R, crandn, gen):
         b, k = 128, 2048
         vol = blob_volume_torch(b, 1001, dev)
         Rp = torch.tensor(rotations(k, 1001), device=dev)
-        # non-FFT bytes: pad x sinc^2 (read b^3, write (2b)^3), extraction (write k (2b)(b+1)),
-        # recentre / crop (read k (2b)^2, write k b^2), all float32 / complex64
-        return (lambda: tt.project_3d_to_2d(vol, Rp)), 4 * b ** 3 + 4 * (2 * b) ** 3 + k * 8 * 2 * b * (b + 1) + \
-            k * 4 * ((2 * b) ** 2 + b * b), \
+        # the map read and the projections written: the padded box and its spectra are the path's own
+        return (lambda: tt.project_3d_to_2d(vol, Rp)), 4 * b ** 3 + 4 * k * b * b, \
             "sinc2_kernel, rows_r2c_kernel, columns_kernel, columns_to_bricks_kernel, extraction, rows_c2r_kernel"
     if name == "backproject":
         b, k = 128, 2048
         imgs = torch.randn((k, b, b), device=dev, generator=gen)
         Rp = torch.tensor(rotations(k, 1002), device=dev)
-        return (lambda: tt.backproject_2d_to_3d(imgs, Rp)), k * 4 * (b * b + (2 * b) ** 2) + k * 8 * 2 * b * (
-            b + 1) + 20 * (2 * b) ** 2 * (b + 1) + 8 * (2 * b) ** 3, \
+        # the images read and the map written
+        return (lambda: tt.backproject_2d_to_3d(imgs, Rp)), 4 * k * b * b + 4 * b ** 3, \
             "rows_r2c_kernel, columns_kernel, insertion, normalize_columns_kernel, rows_c2r_kernel, sinc2_kernel"
     if name == "pack_bricks":
         p = slice_params(n=1, image_shape=(n, n, n), volume=V, rotation=R)
