@@ -56,10 +56,10 @@ __host__ inline int tiles_t(int img_h, int wr) {
     return ((wr + TX - 1) / TX) * ((img_h + TY - 1) / TY);
 }
 
-// The extraction instantiations keep six blocks resident (40 registers, no
-// spills): 389K CTF slices of 32 volumes in 63.9 / 71.7 ms (8 x 32 / 16 x 16
-// tiles) against 65.8 / 74.7 ms at five (47 registers) and 72.8 / 83.1 ms at
-// four.  The insertion's keep five (44 registers; equal times).
+// The extraction instantiations keep six blocks resident (40 registers, 12 to 16
+// bytes of spill stores): 389K CTF slices of 32 volumes in 63.9 / 71.7 ms (8 x
+// 32 / 16 x 16 tiles) against 65.8 / 74.7 ms at five and 72.8 / 83.1 ms at four,
+// when the choice was made.  The insertion's keep five (48 registers).
 template <int TX, bool INSERT, typename VT>
 __global__ void __launch_bounds__(256, INSERT ? 5 : 6)
 batched_slices_kernel(const __grid_constant__ BatchParams bp, unsigned long long* __restrict__ queue,

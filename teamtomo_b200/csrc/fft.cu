@@ -22,12 +22,12 @@
 // A library transform of the padded arrays moves the zeros and the cropped
 // samples through HBM in every pass and needs separate passes for the padding,
 // the scaling and the layouts.  Measured on a B200, whole calls with the
-// library transforms / here: 64^3 x 100 projections 102 / 68 us, 90^3 x 256
-// with both gradients 1060 / 375 us, two 160^3 maps x 400 2680 / 1070 us,
-// 10,000 images of 128^2 (the insertion takes 8.5 ms of it) 13.4 / 10.7 ms.
+// library transforms / here: 64^3 x 100 projections 102 / 59 us, 90^3 x 256
+// with both gradients 1021 / 343 us, two 160^3 maps x 400 2684 / 883 us,
+// 10,000 images of 128^2 (the insertion takes 7.1 ms of it) 13.4 / 9.1 to 9.5 ms.
 // Passes of radix 8, 4, 2 and odd primes through shared memory with a barrier
 // each took 1.58 (rows) and 2.16 ms (columns) of the last, the passes in
-// registers 0.67 and 1.00 ms, at floors of 0.30 and 0.61 ms of HBM traffic:
+// registers 0.63 and 1.00 ms, at floors of 0.30 and 0.61 ms of HBM traffic:
 // the kernels are bound by instruction issue (about 50 per sample) at four
 // blocks' registers per SM.  Sampling the slices in the column kernel took
 // longer than the extraction and the transform one after the other (990 / 800

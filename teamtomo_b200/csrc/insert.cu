@@ -68,7 +68,7 @@ insert_accumulate_kernel(const typename Acc<R>::C* __restrict__ img, const void*
 }
 
 // The same into the bricked float accumulator.  Six resident blocks (40
-// registers, no spills): 1.50 against 1.53 ms at five (256^3 x 2048).
+// registers, 8 bytes of spill stores): 1.50 against 1.53 ms at five (256^3 x 2048).
 __global__ void __launch_bounds__(kTileThreads, 6)
 insert_bricked_kernel(const float2* __restrict__ img, const void* __restrict__ rot, float4* __restrict__ acc,
                       SliceGeom g, int phase, int nphase) {

@@ -3,7 +3,8 @@
 // insert_central_slices_rfft_3d_multichannel, _insert_central_slices_rfft_3d.py:109-210):
 // c volumes share one set of rotations, so each pixel's geometry (rotation,
 // redirect, coordinates, corners and weights) is computed once and applied to
-// every channel.  Layouts: volumes (c, d, h, w/2+1), slices (n, c, h, w/2+1)
+// every channel (but in the insertion's splat, which goes channel by channel:
+// insert.cu).  Layouts: volumes (c, d, h, w/2+1), slices (n, c, h, w/2+1)
 // (the reference's (..., c, h, w) order), insertion accumulators
 // (c, d, h, w/2+1) float4 slots with the weights in channel 0.
 #include <cuda_runtime.h>

@@ -15,8 +15,9 @@ bit-identical to the plain layout:
   8 x 4 pixels touch fewer lines.  The volume's size (padded to even dims).
 
 Each copy costs one streaming pass over the volume.  Measured on a B200 when
-the layouts were chosen (the kernels have since become faster on all three;
-the bricked forward at 256 takes 1.13; ms, each kernel alone, 4096 slices, 2048 at 320; plain / x-paired / bricked):
+the layouts were chosen (ms, each kernel alone, 4096 slices, 2048 at 320;
+plain / x-paired / bricked; the kernels have since become faster on all three,
+the bricked forward at 256 takes 1.13 to 1.19 ms):
 
     box   extraction           backward (dV + dR)   fused MSE            pack (x-pairs, bricks)
     128   0.46 / 0.41 / 0.38   1.07 / 0.98 / 0.92   1.03 / 0.92 / 0.88   0.010, 0.010

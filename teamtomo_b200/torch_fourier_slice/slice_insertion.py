@@ -261,7 +261,7 @@ def _insert(images, R, volume_shape, fftfreq_max, zyx_matrices, deterministic, u
     c = images.shape[1]
     c128 = images.dtype == torch.complex128
     if c > 1 and not c128 and not deterministic:
-        # one geometry pass per pixel for all channels
+        # one call, channel after channel into accumulators back to back
         acc = new_accumulator(volume_shape, False, images.device, channels=c)
         insert_accumulate_multichannel(_lib.dense(images), R, volume_shape, acc, fftfreq_max, zyx_matrices, unshifted)
         return insert_finalize(acc, False)
