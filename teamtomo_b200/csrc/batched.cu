@@ -132,8 +132,9 @@ batched_slices_kernel(const __grid_constant__ BatchParams bp, unsigned long long
             }
         } else {
             for (int first = 0; first < txt; first += 32) {
-                // z-phased filling of large accumulators (the same tiles in every warp)
-                unsigned todo = phase_tiles<TX>(bv.g, m, ty * TY + TY / 2, first, txt, phase, nphase);
+                // z-phased filling of large accumulators, patches within the resolution limit
+                unsigned todo = phase_tiles<TX>(bv.g, m, ty * TY + TY / 2, first, txt, phase, nphase) &
+                                limit_tiles<TX, RPW>(bv.g, iy - lane / TX, first);
                 for (; todo; todo &= todo - 1) {
                     const int ix = (first + __ffs(todo) - 1) * TX + (lane % TX);
                     const bool has_pixel = ix < bv.g.wr && iy < bv.g.img_h;

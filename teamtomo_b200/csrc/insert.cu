@@ -68,7 +68,7 @@ insert_accumulate_kernel(const typename Acc<R>::C* __restrict__ img, const void*
 }
 
 // The same into the bricked float accumulator.  Six resident blocks (40
-// registers, 8 bytes of spill stores): 1.50 against 1.53 ms at five (256^3 x 2048).
+// registers, no spills): 1.50 against 1.53 ms at five (256^3 x 2048).
 __global__ void __launch_bounds__(kTileThreads, 6)
 insert_bricked_kernel(const float2* __restrict__ img, const void* __restrict__ rot, float4* __restrict__ acc,
                       SliceGeom g, int phase, int nphase) {
@@ -86,7 +86,8 @@ insert_bricked_kernel(const float2* __restrict__ img, const void* __restrict__ r
     const SliceRow row = slice_row_geom(g, m, iy);
     const float2* irow = img + (s * g.slice_rows + slice_row(g, iy)) * (int64_t)g.slice_pitch;
     for (int first = 0; first < tx_tiles; first += 32) {
-        unsigned todo = phase_tiles<kTileX>(g, m, ty * kTileY + kTileY / 2, first, tx_tiles, phase, nphase);
+        unsigned todo = phase_tiles<kTileX>(g, m, ty * kTileY + kTileY / 2, first, tx_tiles, phase, nphase) &
+                        limit_tiles<kTileX, 4>(g, iy - (lane >> 3), first);
         for (; todo; todo &= todo - 1) {
             const int ix = (first + __ffs(todo) - 1) * kTileX + (lane & 7);
             float re, im, wscale, c[3];
